@@ -452,7 +452,8 @@ __device__ __forceinline__ void pair_loop(const KArgs& A, double* slot_store, in
     }
     // requests of the steps that complete rows, contiguous in the ring
     const unsigned wants = __ballot_sync(FULL, want);
-    if (dense) {  // every lane has read its request
+    if (dense) {
+      __syncwarp();  // every lane has read its request before the slots are reused
       qhead = (qhead + nround) & (QS - 1);
       qcount -= nround;
     }

@@ -128,3 +128,38 @@ def test_pair_machine_against_first_order(n, planar):
     d = np.abs(a - b).max(axis=(1, 2))
     assert (na == nb).mean() >= 0.98
     assert np.median(d) < 1e-12 and d.max() < 1e-6, (np.median(d), d.max())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("n", [32, 63, 2000])
+def test_requests_reuse_the_ring(n):
+    """Output times in every step: the warp's 64 request slots are reused many
+    times over, and every row is the one of the entry point without a ring
+    (its lanes run their own dense stages; a torn request would show at once).
+    The same arithmetic either way, so rounding of a few ulp is allowed."""
+    import ctypes
+
+    import torch
+
+    import galpy_b200 as gb
+    from galpy_b200 import _lib
+    from test_zz_no_alloc import _launch, _workload
+
+    pot = gb.MWPotential2014()
+    buf, ncomp = gb.compile_potential(pot)
+    w, t = _workload(n)
+    t = np.linspace(0.0, 1.0, 401)[None, :] * t[:, -1:]
+    comps, w0, td = (torch.from_numpy(np.ascontiguousarray(a)).cuda() for a in (buf, w, t))
+    got = []
+    for entry in ("galpy_cuda_integrate_device", "galpy_cuda_integrate_device_noalloc"):
+        out = torch.full((6, 401, n), float("nan"), dtype=torch.float64, device="cuda")
+        err = torch.full((n,), -99, dtype=torch.int32, device="cuda")
+        ns = torch.empty(n, dtype=torch.int64, device="cuda")
+        L = _launch(comps, ncomp, w0, td, out, err, ns, gb.signature(pot), 1)
+        L.comps_host = buf.ctypes.data
+        assert getattr(_lib.lib(), entry)(ctypes.byref(L)) == 0, _lib.last_error()
+        torch.cuda.synchronize()
+        assert not err.any()
+        got.append((out, ns))
+    assert torch.equal(got[0][1], got[1][1])
+    assert float((got[0][0] - got[1][0]).abs().max()) < 1e-13
