@@ -447,13 +447,12 @@ int run_fused(long long n, int nt, const double* t, const double* rows, int nq, 
   cudaError_t e;
   const size_t fbytes = (size_t)(1 + kFactors) * nt * sizeof(double);
   auto kernel = indiv_q ? fused_kernel<NV, false> : fused_kernel<NV, true>;
-  if (bytes > 40 * 1024 &&
-      (e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)bytes)) != cudaSuccess)
-    return fail("interpolation kernel: ", e);
-  if (fbytes > 40 * 1024 &&
+  // the limit belongs to the kernel, not to this launch: always the same one,
+  // so that host threads with other grids do not lower it under each other
+  if ((e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                (int)kFusedMost)) != cudaSuccess ||
       (e = cudaFuncSetAttribute(factor_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)fbytes)) != cudaSuccess)
+                                (int)kFusedMost)) != cudaSuccess)
     return fail("interpolation kernel: ", e);
   if ((e = cudaMallocFromPoolAsync((void**)&f, kFactors * nt * sizeof(double), pool, s)) !=
       cudaSuccess)

@@ -61,3 +61,37 @@ def test_output_over_the_rows():
     out = rows.view(-1)[: n * nq * 6].view(n, nq, 6)
     interpolate_device(rows, td, tq, out)
     assert float((out - ref).abs().max()) < 1e-13
+
+
+def test_threads_with_different_grids():
+    """Host threads on streams of their own, with grids whose blocks need
+    different amounts of shared memory: no call's launch may depend on what
+    another asked of the kernel."""
+    import threading
+
+    import torch
+
+    from galpy_b200.orbit_quantities import interpolate_device
+
+    failed = []
+
+    def work(nt, calls):
+        t = np.linspace(0.0, 0.05 * (nt - 1), nt)
+        rows = torch.from_numpy(_rows(1, t, 6, 3)).cuda()
+        td, tq = torch.from_numpy(t).cuda(), torch.linspace(0.0, t[-1], 8, dtype=torch.float64).cuda()
+        out = torch.empty((1, 8, 6), dtype=torch.float64, device="cuda")
+        torch.cuda.synchronize()
+        stream = torch.cuda.Stream()
+        try:
+            for _ in range(calls):
+                interpolate_device(rows, td, tq, out, stream=stream)
+        except Exception as e:  # noqa: BLE001 (the other thread must end too)
+            failed.append((nt, str(e)))
+        torch.cuda.synchronize()
+
+    threads = [threading.Thread(target=work, args=(nt, 4000)) for nt in (801, 601, 1201, 901)]
+    for th in threads:
+        th.start()
+    for th in threads:
+        th.join()
+    assert not failed, failed
