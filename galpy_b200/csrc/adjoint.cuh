@@ -834,7 +834,7 @@ GPC_HD GPC_FI void mw14_vjp(const GpComp* __restrict__ comp, const double* q, co
     if (!PLANAR)
       mu[PLANAR ? 0 : 2] += amp * (w * sz * z - (sz - a * z2 * izb * izb * izb) * iD3 * lz);
     // da/ds: dD^(-3/2)/ds = -3 s D^(-5/2); ds/da = 1, ds/db = b / zeta
-    const double ds = amp * (s * w - iD3 * izb * zl), bz = b2 * rsqrt_nr(b2) * izb;
+    const double ds = amp * (s * w - iD3 * izb * zl), bz = sqrt(b2) * izb;
     g[2] -= iD3 * B;
     g[3] += ds;
     g[4] += bz * (ds + amp * iD3 * s * izb * izb * zl);

@@ -383,6 +383,31 @@ extern "C" int harness_adj_param_vjp(int planar, int n, const double* x, const d
   return np;
 }
 
+// MWPotential2014's one-pass forms at n points q with vectors l ([n][D]): the
+// acceleration and K l of mw14_tangent, and mw14_vjp's K l and parameter
+// derivatives g [n][7].
+extern "C" int harness_mw14_forms(int planar, int n, const double* q, const double* l,
+                                  const double* pot_args, double* acc, double* Kl, double* mu,
+                                  double* g)
+{
+  const int pot_type[3] = {T_PSWC, T_MN, T_NFW}, D = planar ? 2 : 3;
+  AdjPot P(planar, 3, pot_type, pot_args);
+  if (P.rc) return P.rc;
+  const GpComp* c = P.comps.data();
+  for (int i = 0; i < n; i++) {
+    const size_t o = (size_t)i * D;
+    for (int p = 0; p < 7; p++) g[(size_t)i * 7 + p] = 0.0;
+    if (planar) {
+      mw14_tangent<true>(c, q + o, l + o, acc + o, Kl + o);
+      adj::mw14_vjp<true>(c, q + o, l + o, mu + o, g + (size_t)i * 7);
+    } else {
+      mw14_tangent<false>(c, q + o, l + o, acc + o, Kl + o);
+      adj::mw14_vjp<false>(c, q + o, l + o, mu + o, g + (size_t)i * 7);
+    }
+  }
+  return 0;
+}
+
 // Forward pass per orbit (w0, yT: [nobj][nv]); hrec [nobj][hcap] (may be
 // NULL); nsteps, err [nobj].
 extern "C" int harness_adj_forward(int planar, int nobj, const double* w0, double t0, double T,

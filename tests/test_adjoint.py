@@ -49,6 +49,46 @@ def test_param_derivatives_match_force_differences(harness, golden, name, planar
     assert np.all(np.abs(g - fd) <= 1e-7 * scale + 1e-12), np.abs(g - fd).max(0) / scale
 
 
+@pytest.mark.parametrize("change", ["none", "alpha0", "alpha2.9", "rc/10", "rc*10", "no bulge",
+                                    "no disk", "no halo", "a*10", "b=0"])
+@pytest.mark.parametrize("planar", [False, True])
+def test_mw14_one_pass_forms(harness, golden, planar, change):
+    """MWPotential2014's force, tidal product and parameter derivatives in one
+    pass (variational runs, gradients) against the general forms, away from
+    the usual parameters too.  Both sides lose what the halo's differences
+    cancel: at most (a/r)^2 < 2e4 roundings of 1e-16 here."""
+    if planar and change == "b=0":
+        pytest.skip("the force is singular all over the plane")
+    pt = golden["mw14_planar_type" if planar else "mw14_type"]
+    pa = np.array(golden["mw14_planar_args" if planar else "mw14_args"], float)
+    d = 3 if planar else 5  # the disk's arguments follow the bulge's
+    k, v = {"none": (0, pa[0]), "alpha0": (1, 0.0), "alpha2.9": (1, 2.9), "rc/10": (2, pa[2] / 10),
+            "rc*10": (2, pa[2] * 10), "no bulge": (0, 0.0), "no disk": (d, 0.0),
+            "no halo": (d + 3, 0.0), "a*10": (d + 4, pa[d + 4] * 10), "b=0": (d + 2, 0.0)}[change]
+    pa[k] = v
+    rng = np.random.default_rng(4)
+    n, D = 64, 2 if planar else 3
+    R, ph = np.exp(rng.uniform(np.log(0.3), np.log(30.0), n)), rng.uniform(0, 2 * np.pi, n)
+    q = np.stack([R * np.cos(ph), R * np.sin(ph), 0.3 * R * rng.normal(size=n)], 1)
+    lam = rng.normal(size=(n, 3))
+    if planar:
+        q[:, 2] = lam[:, 2] = 0.0
+    acc, tid, _ = harness.forces(*q.T, pt, pa, planar=planar)
+    K = tid[:, [0, 1, 3, 1, 2, 4, 3, 4, 5]].reshape(n, 3, 3)[:, :D, :D]
+    want = {"acc": acc[:, :D], "Kl": np.einsum("nij,nj->ni", K, lam[:, :D])}
+    want["mu"] = want["Kl"]
+    want["g"] = harness.adj_param_vjp(*q.T, lam, pt, pa, planar=planar)
+    got = {"acc": np.zeros((n, D)), "Kl": np.zeros((n, D)), "mu": np.zeros((n, D)),
+           "g": np.zeros((n, 7))}
+    ptr = lambda a: a.ctypes.data_as(ctypes.POINTER(ctypes.c_double))  # noqa: E731
+    qD, lD = np.ascontiguousarray(q[:, :D]), np.ascontiguousarray(lam[:, :D])
+    assert harness.lib.harness_mw14_forms(int(planar), n, ptr(qD), ptr(lD), ptr(pa),
+                                          *(ptr(got[key]) for key in ("acc", "Kl", "mu", "g"))) == 0
+    for key in want:
+        scale = np.abs(want[key]).max(0 if key == "g" else (0, 1))
+        assert np.all(np.abs(got[key] - want[key]) <= 2e-12 * scale), key
+
+
 def _planar_args(golden, name):
     """(npot, pot_type, pot_args) of the planar form of a golden potential."""
     if name == "mw14":
