@@ -343,8 +343,15 @@ __global__ void __launch_bounds__(kFusedThreads) fused_kernel(long long n, int n
   for (int e = tid; e < nt; e += kFusedThreads) tt[e] = t[e];
   for (int e = tid; e < kFactors * nt; e += kFusedThreads) F[e] = f[e];
   const double* src = rows + i0 * w;
-  for (int o = 0; o < no; o++)
-    for (int e = tid; e < w; e += kFusedThreads) X[o * so + e] = src[(long long)o * w + e];
+  if (w >= kFusedThreads) {
+    for (int o = 0; o < no; o++)
+      for (int e = tid; e < w; e += kFusedThreads) X[o * so + e] = src[(long long)o * w + e];
+  } else {  // an orbit's row would leave threads idle
+    for (int e = tid; e < no * w; e += kFusedThreads) {
+      const int o = e / w;
+      X[o * so + e - o * w] = src[e];
+    }
+  }
   __syncthreads();
   for (int e = tid; e < no * nt; e += kFusedThreads) {
     const int o = e / nt, r = e - o * nt;
@@ -416,9 +423,10 @@ int fail(const char* what, cudaError_t e)
 }
 
 // The fused path's shared memory: with 68 KB (and 5 KB of query weights) a
-// block three blocks fit a multiprocessor; orbits too long for that take one orbit a block up to the
-// largest block, and beyond it the four passes.
+// block three blocks fit a multiprocessor; orbits too long for that take one
+// orbit a block up to the largest block, and beyond it the four passes.
 constexpr size_t kFusedBytes = 68 << 10, kFusedMost = 200 << 10;
+constexpr size_t kSmBytes = 228 << 10;  // of a multiprocessor, 1 KB of it for each block
 
 // Orbits per block of the fused path, its orbit stride and shared bytes;
 // 0 when the grid is too short (its line or parabola needs no moments) or
@@ -436,6 +444,25 @@ int fused_tile(int nt, int* so, size_t* bytes)
   *so = (int)s;
   *bytes = head + tile * per;
   return tile;
+}
+
+// Whether the fused path is the faster one (ns per orbit).  Its solve is a
+// chain of rows for the orbits that a multiprocessor holds at a time, so its
+// time is inverse to their number; long rows leave one or two.  The four
+// passes are bound by memory, and by their own chains when there are few
+// orbits.  Measured, four passes over fused (nv = 6, 100 shared queries):
+// 100,000 orbits of 101 rows 1.83 / 0.85 ms, of 251 rows 3.19 / 2.59; 10,000
+// of 401 rows 0.85 / 0.71, of 501 rows 1.04 / 1.22, of 1,001 rows 1.93 / 4.37;
+// 1,000 of 1,001 rows 1.15 / 0.55.
+template <int NV>
+bool fused_pays(long long n, int nt, int nq, int indiv_q, int tile, size_t bytes)
+{
+  const size_t block = bytes + (indiv_q ? 0 : kQueryChunk * sizeof(QueryWeights)) + 1024;
+  const double held = (double)tile * (double)(kSmBytes / block);
+  const double fused = nt * (0.36 / held + 0.04);
+  const double four =
+      nt * (0.0125 * NV + 1000.0 / (double)n) + (double)nq * NV * (indiv_q ? 0.08 : 0.013);
+  return fused <= four;
 }
 
 template <int NV>
@@ -487,9 +514,22 @@ int run(long long n, int nt, const double* t, int indiv_t, const double* rows, i
   if (!indiv_t && (rows_end <= out || out_end <= rows)) {
     int so = 0;
     size_t bytes = 0;
-    const int tile = fused_tile<NV>(nt, &so, &bytes);
-    if (tile > 0 && (n + tile - 1) / tile < (1LL << 31))
+    int tile = fused_tile<NV>(nt, &so, &bytes);
+    if (tile > 0 && fused_pays<NV>(n, nt, nq, indiv_q, tile, bytes) &&
+        (n + tile - 1) / tile < (1LL << 31)) {
+      // few orbits: smaller tiles, so that every multiprocessor has its three
+      // blocks (1,000 orbits of 4 rows, 1,000 queries: 6 blocks took 0.30 ms)
+      int dev = 0, nsm = 0;
+      if ((e = cudaGetDevice(&dev)) != cudaSuccess ||
+          (e = cudaDeviceGetAttribute(&nsm, cudaDevAttrMultiProcessorCount, dev)) != cudaSuccess)
+        return fail("interpolation: ", e);
+      const long long spread = (n + 3 * nsm - 1) / (3 * nsm);
+      if (spread < tile) {
+        bytes -= (size_t)(tile - spread) * 2 * so * sizeof(double);
+        tile = (int)spread;
+      }
       return run_fused<NV>(n, nt, t, rows, nq, tq, indiv_q, out, tile, so, bytes, pool, s);
+    }
   }
   const long long ncp = indiv_t ? n : 1;
   const size_t vals = (size_t)NV * nt * n;
