@@ -1553,19 +1553,26 @@ int galpy_cuda_accel_device(const void* comps, int ncomp, const int* group, int 
   } else if (precision == GALPY_CUDA_F32BULGE) {
     accel_kernel<MW14MixedPot<false, MIX_F32BULGE>, PREC_FP64>
         <<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc);
+  } else if (mw14 && !group) {  // one potential: the integrations' tabulated radial force
+    cudaMemPool_t pool = nullptr;
+    const int rc = library_pool(&pool);
+    if (rc) return rc;
+    void* rtab = nullptr;
+    GPC_CUDA_TRY(alloc_async(&rtab, kRadBytes, pool, s));
+    build_radial(c, rtab, s);
+    const double* tab = static_cast<const double*>(rtab);
+    if (precision == GALPY_CUDA_FP64)
+      accel_kernel<RadialPot<false>, PREC_FP64>
+          <<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc, tab);
+    else
+      accel_kernel<RadialPot<false>, PREC_F32>
+          <<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc, tab);
+    cudaFreeAsync(rtab, s);
   } else if (precision == GALPY_CUDA_FP64) {
-    if (mw14 && !group) {  // one potential: the integrations' tabulated radial force
-      void* rtab = nullptr;
-      GPC_CUDA_TRY(cudaMallocAsync(&rtab, kRadBytes, s));
-      build_radial(c, rtab, s);
-      accel_kernel<RadialPot<false>, PREC_FP64><<<blocks, 256, 0, s>>>(
-          c, ncomp, group, planar, pos, n, acc, static_cast<const double*>(rtab));
-      cudaFreeAsync(rtab, s);
-    } else if (mw14) {
+    if (mw14)
       accel_kernel<MW14GroupPot, PREC_FP64><<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc);
-    } else {
+    else
       accel_kernel<DynPot, PREC_FP64><<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc);
-    }
   } else {
     if (mw14)
       accel_kernel<MW14GroupPot, PREC_F32><<<blocks, 256, 0, s>>>(c, ncomp, group, planar, pos, n, acc);

@@ -221,9 +221,11 @@ int integrateOrbit_dxdv_batch_cuda(int planar, int nobj, double *yo, int nt, dou
                                    int odeint_type, const galpy_cuda_opts *opts);
 
 /* Device-pointer entry point: all arrays live on the device, the call is
- * asynchronous on `stream`.  Needs 64 bytes of device scratch for the
- * work-stealing counter (plus the scheduling scratch, see `schedule`),
- * allocated stream-ordered per call. */
+ * asynchronous on `stream`.  Its scratch is allocated stream-ordered per call
+ * from the device's default pool: 128 bytes of control words, the scheduling
+ * scratch (see `schedule`), dop853's dense-output requests (22 KB for each
+ * resident warp) and, for MWPotential2014 as one potential with comps_host
+ * set, the table of its radial force (246 KB). */
 typedef struct galpy_cuda_launch {
   int planar, variational, odeint_type, precision;
   long long nobj;
@@ -405,7 +407,12 @@ int galpy_cuda_adjoint_params(int planar, int npot, const int *pot_type, const d
  * (galpy's evaluateRforces/zforces in Cartesian form; the acceleration that
  * evalRectForce, integrateFullOrbit.c:1307, hands to the steppers).
  * signature GALPY_CUDA_SIG_MW14 selects the compile-time MWPotential2014
- * path of the integration kernels; precision as galpy_cuda_opts.
+ * path of the integration kernels; precision as galpy_cuda_opts.  With that
+ * signature, no group, and a float64 or float32 force (GALPY_CUDA_FP64,
+ * _F32FORCE, _F32FORCE_DF) the call tabulates the potential's radial force
+ * first, as a launch does: 246 KB allocated stream-ordered from the library's
+ * private memory pool (kept for the next call; galpy_cuda_trim_memory
+ * returns it).  Every other form allocates nothing.
  * Asynchronous on `stream`. */
 int galpy_cuda_accel_device(const void *comps, int ncomp, const int *group, int planar,
                             int signature, int precision, const double *pos, long long n,

@@ -40,15 +40,18 @@ def _points(lo, hi, n, planar, seed):
     return np.stack([R * np.cos(ph), R * np.sin(ph), z])
 
 
-def _errors(P, planar, signature):
-    """Force errors over 2^-53 |force|."""
+def _errors(P, planar, signature, change=None):
+    """Force errors over 2^-53 |force|; change: {argument: value}, the disk's
+    and halo's arguments counted from 3."""
     import torch
 
     import galpy_b200 as gb
 
-    pot = gb.MWPotential2014()
-    buf, n = gb.compile_potential(pot, planar=planar)
-    _, _, pa = gb.parse_pot(pot, planar=planar)
+    _, pt, pa = gb.parse_pot(gb.MWPotential2014(), planar=planar)
+    pa = np.array(pa, float)
+    for k, v in (change or {}).items():
+        pa[k if k < 3 or planar else k + 2] = v
+    buf, n = gb.compile_potential((pt, pa), planar=planar)
     acc = torch.empty((3, P.shape[1]), dtype=torch.float64, device="cuda")
     gb.accel_device(torch.from_numpy(buf).cuda(), n, torch.from_numpy(P).cuda(), acc,
                     planar=planar, signature=signature)
@@ -65,6 +68,19 @@ def _errors(P, planar, signature):
 def test_radial_force_is_closer_than_the_direct_form(lo, hi, planar):
     P = _points(lo, hi, 400, planar, 3)
     rad, direct = _errors(P, planar, 1), _errors(P, planar, 0)
+    assert rad.max() <= BOUND, rad.max()
+    assert np.sqrt((rad ** 2).mean()) <= np.sqrt((direct ** 2).mean())
+
+
+# alpha, rc, the halo's scale, and lists with one spherical component: the
+# table is built from the launch's own parameters (a row's degree suffices for
+# any power law up to r^-3 and for the cutoff at any rc)
+@pytest.mark.parametrize("change", [{1: 0.0}, {1: 2.9}, {2: 0.0237}, {2: 2.37}, {0: 0.0}, {6: 0.0},
+                                    {7: 0.05}, {7: 50.0}])
+@pytest.mark.parametrize("planar", [False, True])
+def test_radial_force_with_other_parameters(change, planar):
+    P = _points(0.01, 300.0, 400, planar, 9)
+    rad, direct = _errors(P, planar, 1, change), _errors(P, planar, 0, change)
     assert rad.max() <= BOUND, rad.max()
     assert np.sqrt((rad ** 2).mean()) <= np.sqrt((direct ** 2).mean())
 
@@ -151,3 +167,49 @@ def test_radial_force_in_single_precision_at_row_edges():
     r2 = np.concatenate([e * (1 - 2.0 ** -22), e, e * (1 + 2.0 ** -22), [2.0 ** -31, 2.0 ** 18, 1e7]])
     err = _kick_errors(np.stack([np.sqrt(r2), 0 * r2, 0 * r2]), False, 1)
     assert err.max() <= BOUND_F32, err.max()
+
+
+def _default_pool_high(reset=False):
+    from cuda.bindings import driver, runtime as rt
+
+    _, pool = rt.cudaDeviceGetDefaultMemPool(0)
+    attr = rt.cudaMemPoolAttr.cudaMemPoolAttrUsedMemHigh
+    if reset:
+        rt.cudaMemPoolSetAttribute(pool, attr, driver.cuuint64_t(0))
+    return int(rt.cudaMemPoolGetAttribute(pool, attr)[1])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "f32force", "f32force_df"])
+@pytest.mark.parametrize("planar", [False, True])
+def test_accelerations_are_the_integrators_own(planar, precision):
+    """accel_device gives the kicks of a leapfrog step of length one from rest
+    (bit for bit in float64; in single precision the two kernels may fuse the
+    radii's sums differently, an ulp of each, which the force's second power
+    of the radius doubles) and takes no memory from the device's default pool."""
+    import torch
+
+    import galpy_b200 as gb
+
+    pot = gb.MWPotential2014()
+    buf, ncomp = gb.compile_potential(pot, planar=planar)
+    sig = gb.signature(pot, planar=planar)
+    P = _points(1e-3, 600.0, 3000, planar, 11)
+    if precision == "f32force_df":  # (positions are rounded to the pairs, too)
+        P = P.astype(np.float32).astype(float)
+    k, n = (2 if planar else 3), P.shape[1]
+    comps, pos = torch.from_numpy(buf).cuda(), torch.from_numpy(P).cuda()
+    acc = torch.zeros((3, n), dtype=torch.float64, device="cuda")
+    torch.cuda.synchronize()
+    before = _default_pool_high(reset=True)
+    gb.accel_device(comps, ncomp, pos, acc, planar=planar, signature=sig, precision=precision)
+    torch.cuda.synchronize()
+    assert _default_pool_high() == before
+    w = torch.zeros((2 * k, n), dtype=torch.float64, device="cuda")
+    w[:k] = pos[:k]
+    out = torch.empty((n, 1, 2 * k), dtype=torch.float64, device="cuda")
+    err = torch.empty(n, dtype=torch.int32, device="cuda")
+    gb.integrate_device(comps, ncomp, w, torch.tensor([0.0, 1.0], dtype=torch.float64, device="cuda"),
+                        out, err, "leapfrog_cuda", planar=planar, out_layout="aos_rect", out_row0=1,
+                        dt=1.0, precision=precision, signature=sig, comps_host=buf)
+    d, mag = (out[:, 0, k:].T - acc[:k]).abs().max(0).values, acc[:k].norm(dim=0)
+    assert float((d / mag).max()) <= (0.0 if precision == "fp64" else 6 * 2.0 ** -24)
