@@ -245,10 +245,13 @@ GPC_HD GPC_FI void eval_force2(const GpComp* comp, int ncomp, const double* q1, 
   } else if constexpr (!VAR && PREC == PREC_FP64 && PairListOf<POT>::value) {
     accel2<double, D == 2, POT>(comp, ncomp, q1, q2, a1, a2, t1, t2);
   } else {
+    bool same = t1 == t2;  // one point given twice: evaluated once (accel2)
+#pragma unroll
+    for (int i = 0; i < NA; i++) same = same && q1[i] == q2[i];
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
-    for (int k = 0; k < 2; k++) {
+    for (int k = 0; k < (same ? 1 : 2); k++) {
       double q[NA], a[NA];
 #pragma unroll
       for (int i = 0; i < NA; i++) q[i] = k ? q2[i] : q1[i];

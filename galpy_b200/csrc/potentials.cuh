@@ -1102,14 +1102,19 @@ struct DynPot {
   }
   // Two points at once (times t1, t2): the usual components and the Dehnen
   // bar side by side; any other component, or a wrapper with the records it
-  // wraps, one point after the other through sum.
+  // wraps, one point after the other through sum (the first one only when
+  // they are the same: q is then not used).
   template <typename T, bool PLANAR>
   GPC_HD GPC_FI static void sum2(const GpComp* __restrict__ comp, int ncomp, PairPoint<T>& p,
-                                 PairPoint<T>& q, double t1, double t2)
+                                 PairPoint<T>& q, double t1, double t2, bool same)
   {
     for (int k = 0; k < ncomp;) {
       const GpComp* cp = comp + k;
       const int type = ldg(&cp->type);
+      if (type == T_PAYLOAD) {  // read by the record before it
+        k++;
+        continue;
+      }
       if (type == T_DEHNENBAR) {
         double ax, ay, az, bx, by, bz;
         dbar_accel<PLANAR>(cp, t1, (double)p.x, (double)p.y, (double)p.z, ax, ay, az);
@@ -1129,19 +1134,37 @@ struct DynPot {
         k++;
         continue;
       }
-      const int n = is_wrapper(type) ? 1 + (int)ldg(&cp->c[15]) : 1;
+      if (type == T_SCF) {
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
-      for (int j = 0; j < 2; j++) {
-        PairPoint<T> u = j ? q : p;
+        for (int j = 0; j < (same ? 1 : 2); j++) {
+          const ScfAcc f = scf_accel_called<PLANAR>(cp, (double)(j ? q.x : p.x),
+                                                    (double)(j ? q.y : p.y),
+                                                    (double)(j ? q.z : p.z));
+          AddAcc<T>& a = j ? q.a0 : p.a0;
+          a.x += T(f.x);
+          a.y += T(f.y);
+          if (!PLANAR) a.z += T(f.z);
+        }
+        k++;
+        continue;
+      }
+      const int n = is_wrapper(type) ? 1 + (int)ldg(&cp->c[15]) : 1;
+      // (the points go through local memory, so that the other one's fifteen
+      // values do not hold registers while one of these larger forces runs)
+      PairPoint<T> pq[2] = {p, q};
+#if defined(__CUDA_ARCH__)
+#pragma unroll 1
+#endif
+      for (int j = 0; j < (same ? 1 : 2); j++) {
+        PairPoint<T> u = pq[j];
         sum<T, PLANAR>(cp, nullptr, n, u.x, u.y, u.z, u.z2, u.R2, u.r2, u.gR, u.gz, u.gyx, u.a0,
                        j ? t2 : t1);
-        if (j)
-          q = u;
-        else
-          p = u;
+        pq[j] = u;
       }
+      p = pq[0];
+      q = pq[1];
       k += n;
     }
   }
@@ -1170,7 +1193,7 @@ struct DynPotCommon {
   // Two points at once; the less usual components one point after the other.
   template <typename T, bool PLANAR>
   GPC_HD GPC_FI static void sum2(const GpComp* __restrict__ comp, int ncomp, PairPoint<T>& p,
-                                 PairPoint<T>& q, double /*t1*/, double /*t2*/)
+                                 PairPoint<T>& q, double /*t1*/, double /*t2*/, bool same)
   {
     for (int k = 0; k < ncomp; k++) {
       const GpComp* cp = comp + k;
@@ -1178,7 +1201,7 @@ struct DynPotCommon {
 #if defined(__CUDA_ARCH__)
 #pragma unroll 1
 #endif
-      for (int j = 0; j < 2; j++) {
+      for (int j = 0; j < (same ? 1 : 2); j++) {
         PairPoint<T> u = j ? q : p;
         comp_accel<T, PLANAR, kRunTimeCommon>(cp, ScalarsGlobal{cp}, u.x, u.y, u.z, u.z2, u.R2,
                                               u.r2, u.gR, u.gz, u.gyx, u.a0, 0.0);
@@ -1486,11 +1509,16 @@ GPC_HD GPC_FI void accel2(const GpComp* __restrict__ comp, int ncomp, const T* q
     const T z2 = PLANAR ? T(0) : z * z;
     p[j] = PairPoint<T>{x, y, z, z2, R2, R2 + z2, T(0), T(0), T(0), {T(0), T(0), T(0)}};
   }
-  POT::template sum2<T, PLANAR>(comp, ncomp, p[0], p[1], t1, t2);
+  // one point given twice (rk6's seventh stage, dop853's sixteenth, the
+  // start-ups): components that go one after the other go once
+  bool same = t1 == t2;
+#pragma unroll
+  for (int k = 0; k < (PLANAR ? 2 : 3); k++) same = same && q1[k] == q2[k];
+  POT::template sum2<T, PLANAR>(comp, ncomp, p[0], p[1], t1, t2, same);
 #pragma unroll
   for (int j = 0; j < 2; j++) {
     T* a = j ? a2 : a1;
-    const PairPoint<T>& u = p[j];
+    const PairPoint<T> u = j && !same ? p[1] : p[0];
     a[0] = u.x * u.gR + u.a0.x;
     a[1] = u.y * (u.gR + u.gyx) + u.a0.y;
     if (!PLANAR) a[2] = u.z * u.gz + u.a0.z;

@@ -755,6 +755,22 @@ GPC_HD inline void scf_accel(const GpComp* __restrict__ cp, double x, double y, 
   az = PLANAR ? 0.0 : -(gr * zz - gth * R);
 }
 
+// scf_accel as a call (device code): its own registers for the sums, whatever
+// its caller holds.
+struct ScfAcc {
+  double x, y, z;
+};
+template <bool PLANAR>
+#if defined(__CUDACC__)
+__host__ __device__ __noinline__
+#endif
+ScfAcc scf_accel_called(const GpComp* __restrict__ cp, double x, double y, double z)
+{
+  ScfAcc r{0.0, 0.0, 0.0};
+  scf_accel<PLANAR>(cp, x, y, z, r.x, r.y, r.z);
+  return r;
+}
+
 // Acceleration and K = -grad grad Phi added to ax.. and K (PLANAR: at
 // z = 0): the spherical second derivatives, then the cylindrical ones by the
 // chain rule through r = sqrt(R^2 + z^2), theta = atan2(R, z) (as the

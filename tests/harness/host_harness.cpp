@@ -298,6 +298,34 @@ extern "C" int harness_forces_at(int planar, int n, const double* x, const doubl
   return 0;
 }
 
+// Two forces at once (eval_force2, the pair machines' call) at points q1, q2
+// ([n][D], [n][2D] with deviations) and times t1, t2: a1, a2 alike.  list: 0
+// the full run-time list, 1 the common one.
+extern "C" int harness_force_pairs(int planar, int var, int list, int n, const double* q1,
+                                   const double* q2, double t1, double t2, int npot,
+                                   const int* pot_type, const double* pot_args, double* a1,
+                                   double* a2)
+{
+  std::vector<GpComp> comps;
+  int rc = records(planar, npot, pot_type, pot_args, comps);
+  if (rc) return rc;
+  const GpComp* c = comps.data();
+  const int nrec = (int)comps.size(), NA = (planar ? 2 : 3) * (var ? 2 : 1);
+  for (int i = 0; i < n; i++) {
+    const size_t o = (size_t)i * NA;
+#define PAIR(D, VAR, POT) \
+  eval_force2<D, PREC_FP64, VAR, POT>(c, nrec, q1 + o, q2 + o, a1 + o, a2 + o, nullptr, t1, t2)
+    if (planar && var) PAIR(2, true, DynPot);
+    else if (var) PAIR(3, true, DynPot);
+    else if (planar && list) PAIR(2, false, DynPotCommon);
+    else if (list) PAIR(3, false, DynPotCommon);
+    else if (planar) PAIR(2, false, DynPot);
+    else PAIR(3, false, DynPot);
+#undef PAIR
+  }
+  return 0;
+}
+
 extern "C" int harness_forces(int planar, int n, const double* x, const double* y,
                               const double* z, int npot, const int* pot_type,
                               const double* pot_args, double* acc, double* tidal, double* acc32)

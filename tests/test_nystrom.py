@@ -8,6 +8,7 @@ from fractions import Fraction
 
 import numpy as np
 import pytest
+import timedep_pots
 
 CSRC = os.path.join(os.path.dirname(__file__), "..", "galpy_b200", "csrc")
 
@@ -91,6 +92,60 @@ def test_dop853_controller_root(harness):
     got = _controller(harness, 1, e)
     want = np.clip(e, 1e-9, 1e6) ** -0.125
     assert np.abs(got / want - 1).max() < 8 * 2.0 ** -53
+
+
+PAIR_POTS = ["mw14", "hernquist", "loghalo", "logtri", "power", "plummer", "kks", "einasto", "hh",
+             "kuzmindisk", "ell_trinfw", *timedep_pots.NAMES, *timedep_pots.WRAPPED]
+
+
+@pytest.mark.parametrize("name", PAIR_POTS)
+@pytest.mark.parametrize("planar", [False, True])
+def test_force_pairs(harness, golden, name, planar):
+    """Two forces at once against each alone, in both run-time lists and with
+    deviations: components evaluated side by side and one after the other,
+    continuation records, wrappers with the records they wrap, times of their
+    own, and one point given twice (whose second half is copied)."""
+    import ctypes
+
+    if name == "hh" and not planar:
+        pytest.skip("a planar potential")
+    npot = None
+    if name in timedep_pots.WRAPPED:
+        pt, pa, npot = timedep_pots.wrapped(name, planar=planar)
+    elif name in timedep_pots.NAMES:
+        pt, pa = timedep_pots.potential(name, planar=planar)
+    else:
+        key = name + "_planar" if planar and name + "_planar_type" in golden else name
+        pt, pa = golden[key + "_type"], golden[key + "_args"]
+    pt, pa = np.ascontiguousarray(pt, np.int32), np.ascontiguousarray(pa, float)
+    D, n = (2 if planar else 3), 16
+    rng = np.random.default_rng(8)
+    ptr = lambda a, c=ctypes.c_double: a.ctypes.data_as(ctypes.POINTER(c))  # noqa: E731
+    timed = name in timedep_pots.NAMES + timedep_pots.WRAPPED
+    full_only = timed or name.startswith("ell")  # (the common list leaves those out)
+    for var in (False, True):
+        if var and name.startswith("scf"):
+            continue  # run on the device only
+        for lst in ((0,) if var or full_only else (0, 1)):
+            for q_same, t1, t2 in ((False, 0.3, 0.7), (True, 0.4, 0.4), (True, 0.3, 0.7)):
+                NA = 2 * D if var else D
+                q1 = np.concatenate([rng.uniform(0.3, 1.5, (n, D)), rng.normal(size=(n, NA - D))], 1)
+                q2 = q1.copy() if q_same else q1 + rng.uniform(0.1, 0.2, q1.shape)
+                a1, a2 = np.zeros_like(q1), np.zeros_like(q1)
+                assert harness.lib.harness_force_pairs(
+                    int(planar), int(var), lst, n, ptr(q1), ptr(q2), ctypes.c_double(t1),
+                    ctypes.c_double(t2), len(pt) if npot is None else npot, ptr(pt, ctypes.c_int),
+                    ptr(pa), ptr(a1), ptr(a2)) == 0
+                for q, t, a in ((q1, t1, a1), (q2, t2, a2)):
+                    z = q[:, 2] if D == 3 else np.zeros(n)
+                    acc, tid, _ = harness.forces(q[:, 0], q[:, 1], z, pt, pa, planar=planar, t=t,
+                                                 npot=npot)
+                    want = acc[:, :D]
+                    if var:
+                        K = tid[:, [0, 1, 3, 1, 2, 4, 3, 4, 5]].reshape(n, 3, 3)[:, :D, :D]
+                        want = np.concatenate([want, np.einsum("nij,nj->ni", K, q[:, D:])], 1)
+                    # the same sums up to their order: a few roundings
+                    assert np.abs(a - want).max() <= 1e-14 * np.abs(want).max(), (var, lst, t1, t2)
 
 
 @pytest.mark.gpu
