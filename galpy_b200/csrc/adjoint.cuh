@@ -445,8 +445,8 @@ GPC_HD GPC_FI void run_stages(const Field<POT>& F, const double* y, double h, do
 }
 
 // ------------------------------------------- Nystrom stages, in pairs ---
-// Two accelerations at once: compile-time lists side by side, a run-time list
-// one after the other through the same code.
+// Two accelerations at once: compile-time lists side by side, run-time lists
+// component by component.
 template <int D, class POT>
 GPC_HD GPC_FI void accel_pair(const Field<POT>& F, const double* q1, const double* q2, double* a1,
                               double* a2)
@@ -766,7 +766,7 @@ template <int D, class POT>
 GPC_HD void replay_orbit(const Field<POT>& F, const double* w0, double t0, double T,
                          const double* hrec, long long hs, long long nsteps, double* yT)
 {
-  double x[D], v[D], xn[D], vn[D];
+  double x[D], v[D], xn[D];
   Accs<D, 16> a;
   copy<D>(w0, x);
   copy<D>(w0 + D, v);
@@ -784,9 +784,9 @@ GPC_HD void replay_orbit(const Field<POT>& F, const double* w0, double t0, doubl
       final_rows<D, POT>(F, x, v, h, (T - t) / h, a, yT);
       return;
     }
-    dop853_error<D>(a, x, v, xn, h, 1.0, 1.0, vn);  // for the velocity, rounded as the forward pass's
+#pragma unroll
+    for (int i = 0; i < D; i++) v[i] = v[i] + h * dop853_increment(a, i);
     copy<D>(xn, x);
-    copy<D>(vn, v);
     copy<D>(a.v[12], a.v[0]);
     t = t + h;
   }
@@ -1069,11 +1069,7 @@ GPC_HD void backward_orbit(const Field<POT>& F, double T, const double* ck, long
         step_rounds<D, POT>(F, x, v, h, a, xn);
 #pragma unroll
         for (int i = 0; i < D; i++) {
-          double inc = 0.0;
-#pragma unroll
-          for (int k = 0; k < 12; k++)
-            if (k == 0 || k >= 5) inc += GPC_NY.b[k] * a.v[k][i];
-          v[i] += h * inc;
+          v[i] = v[i] + h * dop853_increment(a, i);
           x[i] = xn[i];
           a.v[0][i] = a.v[12][i];
         }

@@ -887,6 +887,18 @@ GPC_HD inline void dop853_force_free(const double* x0, const double* v0, double 
   }
 }
 
+// Component i of the velocity's increment of a step over its size, sum_k b_k
+// a_k; one function, so that every pass that repeats a step (the adjoint's
+// replay and its segments) rounds it alike.
+template <class G>
+GPC_HD GPC_FI double dop853_increment(const G& g, int i)
+{
+  const auto& b = GPC_NY.b;
+  return mad(b[0], g.template a<1>(i), b[5] * g.template a<6>(i)) + b[6] * g.template a<7>(i) +
+         b[7] * g.template a<8>(i) + b[8] * g.template a<9>(i) + b[9] * g.template a<10>(i) +
+         b[10] * g.template a<11>(i) + b[11] * g.template a<12>(i);
+}
+
 // The new velocity vn of a step of size h from (x0, v0) to the position x13,
 // and the step's error norm (leung_dop853.c:390-418); g gives component i of
 // the accelerations a1, a4..a12.
@@ -902,12 +914,10 @@ GPC_HD GPC_FI double dop853_error(const G& g, const double* x0, const double* v0
     const double A6 = g.template a<6>(i), A7 = g.template a<7>(i), A8 = g.template a<8>(i);
     const double A9 = g.template a<9>(i), A10 = g.template a<10>(i), A11 = g.template a<11>(i);
     const double A12 = g.template a<12>(i);
-    const auto& b = GPC_NY.b;
     const auto& ev = GPC_NY.ev;
     const auto& ex = GPC_NY.ex;
     const auto& hx = GPC_NY.hx;
-    const double inc = mad(b[0], A1, b[5] * A6) + b[6] * A7 + b[7] * A8 + b[8] * A9 + b[9] * A10 +
-                       b[10] * A11 + b[11] * A12;
+    const double inc = dop853_increment(g, i);
     vn[i] = v0[i] + h * inc;
     const double isv = rcp_nr(atol + rtol * dmax(fabs(v0[i]), fabs(vn[i])));
     const double isx = rcp_nr(atol + rtol * dmax(fabs(x0[i]), fabs(x13[i])));
