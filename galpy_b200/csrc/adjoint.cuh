@@ -390,60 +390,6 @@ struct Field {
   const double* scal;
 };
 
-template <bool PLANAR, class POT>
-GPC_HD GPC_NI V3 accel_at(const GpComp* __restrict__ comp, int ncomp, const double* scal,
-                          double x, double y, double z)
-{
-  V3 a = {0.0, 0.0, 0.0};
-  accel<double, PLANAR, POT>(comp, ncomp, x, y, z, a.x, a.y, a.z, scal);
-  return a;
-}
-
-// k = f(Y) = (velocities, accelerations); state (x, y[, z], vx, vy[, vz]).
-template <int D, class POT>
-GPC_HD GPC_FI void rhs(const Field<POT>& F, const double* Y, double* k)
-{
-  const V3 a = accel_at<D == 2, POT>(F.comp, F.ncomp, F.scal, Y[0], Y[1],
-                                     D == 3 ? Y[D - 1] : 0.0);
-#pragma unroll
-  for (int c = 0; c < D; c++) k[c] = Y[D + c];
-  k[D] = a.x;
-  k[D + 1] = a.y;
-  if (D == 3) k[2 * D - 1] = a.z;
-}
-
-// The first-order form of a step, the independent one that the tests rebuild
-// checkpoints with: stages I0..I1-1 from y with step h (k[0..I0-1] given).  Q,
-// if not null, receives the stage positions.
-template <int D, class POT, int I0, int I1>
-GPC_HD GPC_FI void run_stages(const Field<POT>& F, const double* y, double h, double (*k)[2 * D],
-                              double (*Q)[D])
-{
-  constexpr int N = 2 * D;
-#pragma unroll
-  for (int i = I0; i < I1; i++) {
-    double acc[N];
-#pragma unroll
-    for (int c = 0; c < N; c++) acc[c] = 0.0;
-#pragma unroll
-    for (int j = 0; j < i; j++) {
-      const double a = A(i, j);
-      if (a != 0.0) {
-#pragma unroll
-        for (int c = 0; c < N; c++) acc[c] += a * k[j][c];
-      }
-    }
-    double Y[N];
-#pragma unroll
-    for (int c = 0; c < N; c++) Y[c] = y[c] + h * acc[c];
-    if (Q) {
-#pragma unroll
-      for (int c = 0; c < D; c++) Q[i][c] = Y[c];
-    }
-    rhs<D, POT>(F, Y, k[i]);
-  }
-}
-
 // ------------------------------------------- Nystrom stages, in pairs ---
 // Two accelerations at once: compile-time lists side by side, run-time lists
 // component by component.
@@ -598,21 +544,6 @@ GPC_HD void hinit(const Field<POT>& F, const double* x, const double* v, double*
   const double h1 = pow(0.01 / der12, 1.0 / 8.0);
   c.h = csign(dmin(100.0 * fabs(c.h), dmin(fabs(h1), fabs(c.hmax))), c.pos_neg);
   begin_attempt(c);
-}
-
-// The new state of a first-order step, y + h sum_j b_j k_j, in the
-// reference's order of summation; also returns the combined increment.
-template <int D>
-GPC_HD GPC_FI void new_state(const double* y, double h, const double (*k)[2 * D], double* inc,
-                             double* ynew)
-{
-  using namespace dp;
-#pragma unroll
-  for (int i = 0; i < 2 * D; i++) {
-    inc[i] = b1 * k[0][i] + b6 * k[5][i] + b7 * k[6][i] + b8 * k[7][i] + b9 * k[8][i] +
-             b10 * k[9][i] + b11 * k[10][i] + b12 * k[11][i];
-    ynew[i] = y[i] + h * inc[i];
-  }
 }
 
 // The controller's decision on an attempt with error norm e

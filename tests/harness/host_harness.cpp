@@ -518,6 +518,33 @@ extern "C" int harness_adj_gradient(int planar, int nobj, const double* w0, doub
 }
 
 namespace {
+// A DOP853 step of size h in its first-order form, from y to ynew: stages with
+// state (x, v) and derivative k = (v, a), the reference's order of summation.
+// Independent of the engine's second-order form.
+template <int D>
+void first_order_step(const AdjPot& P, const double* y, double h, double (*k)[2 * D], double* ynew)
+{
+  constexpr int N = 2 * D;
+  for (int i = 0; i < 12; i++) {
+    double Y[N];
+    for (int c = 0; c < N; c++) {
+      double acc = 0.0;
+      for (int j = 0; j < i; j++)
+        if (adj::A(i, j) != 0.0) acc += adj::A(i, j) * k[j][c];
+      Y[c] = i ? y[c] + h * acc : y[c];
+    }
+    double az = 0.0;
+    accel<double, D == 2, DynPot>(P.comps.data(), (int)P.comps.size(), Y[0], Y[1],
+                                  D == 3 ? Y[2] : 0.0, k[i][D], k[i][D + 1], az);
+    if (D == 3) k[i][N - 1] = az;
+    for (int c = 0; c < D; c++) k[i][c] = Y[D + c];
+  }
+  using namespace dp;
+  for (int c = 0; c < N; c++)
+    ynew[c] = y[c] + h * (b1 * k[0][c] + b6 * k[5][c] + b7 * k[6][c] + b8 * k[7][c] + b9 * k[8][c] +
+                          b10 * k[9][c] + b11 * k[10][c] + b12 * k[11][c]);
+}
+
 // Checkpoints of the frozen-step map (state and time at each segment start,
 // the step sizes), then the device's backward sweep.
 template <int D>
@@ -526,7 +553,7 @@ void backward_frozen(const AdjPot& P, const double* w0, double t0, double T, con
 {
   constexpr int N = 2 * D, CW = N + 1 + adj::kCkptEvery;
   std::vector<double> ck((size_t)((ns + adj::kCkptEvery - 1) / adj::kCkptEvery + 1) * CW);
-  double y[N], k[12][N], inc[N], ynew[N], t = t0;
+  double y[N], k[12][N], ynew[N], t = t0;
   for (int c = 0; c < N; c++) y[c] = w0[c];
   for (long long n = 0; n < ns; n++) {
     double* p = ck.data() + (n / adj::kCkptEvery) * CW;
@@ -535,9 +562,7 @@ void backward_frozen(const AdjPot& P, const double* w0, double t0, double T, con
       p[N] = t;
     }
     p[N + 1 + n % adj::kCkptEvery] = h[n];
-    adj::rhs<D, DynPot>(P.field(), y, k[0]);
-    adj::run_stages<D, DynPot, 1, 12>(P.field(), y, h[n], k, nullptr);
-    adj::new_state<D>(y, h[n], k, inc, ynew);
+    first_order_step<D>(P, y, h[n], k, ynew);
     for (int c = 0; c < N; c++) y[c] = ynew[c];
     t = t + h[n];
   }
