@@ -11,8 +11,9 @@ how ragged the step counts are):
   holds two warps whatever the block, and blocks of 96 -- which a sample of
   the batching workload preferred -- left 6 warps per SM and made the full
   batch 22 % slower);
-* ``variant`` -- register budget: 0 = compiler default (up to 255 registers
-  a thread), 1 = capped so that more blocks are resident per SM;
+* ``variant`` -- register budget: 0 = the kernel's default (up to 255 registers
+  a thread, less where more resident blocks pay), 1 = capped so that more
+  blocks are resident per SM; timed once where both are the same kernel;
 * ``schedule`` -- not tuned: always longest first by the estimated cost
   |t_end - t_0| * orbital frequency.  Its pre-pass costs about a millisecond,
   and what it prevents -- the longest orbits starting late and running alone
@@ -34,7 +35,7 @@ import os
 import threading
 
 from . import _lib
-from .integrate import integrate_device, parse_integrator
+from .integrate import _precision, integrate_device, parse_integrator
 
 _lock = threading.Lock()
 _memo = {}
@@ -147,6 +148,12 @@ def tune(comps, ncomp, w0, t, out, err, int_method, planar=False, variational=Fa
 
     results = []
     cands = candidates(int_method)
+    # variational runs have one kernel; with the tabulated radial force the
+    # capped one is the default (orbit_kernel.cuh) but for rk6 and dop853
+    radial = signature == 1 and group is None and comps_host is not None and \
+        _precision(precision) in (_lib.FP64, _lib.F32FORCE, 4)
+    if variational or (radial and parse_integrator(int_method) not in (2, 6)):
+        cands = [c for c in cands if c["variant"] == 0]
     run(cands[0])  # warm-up: module load, first-touch of the buffers
     for cfg in cands:
         e0, e1 = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
