@@ -556,7 +556,8 @@ def main():
                                     "(galpy_cuda_fp64_peak); MEASURED_PEAKS.json has no FP64 "
                                     "figure"},
         "clocks": clk,
-        "gpu_launches": 2 * args.steps,  # cost_kernel + orbit_kernel per graph replay
+        # cost_kernel + radial_table_kernel + orbit_kernel per graph replay
+        "gpu_launches": 3 * args.steps,
     }
 
     # energy drift of the headline run (initial state vs final snapshot)
@@ -659,7 +660,7 @@ def interp_leg(gb, torch, dev, stream, pg, n=1 << 20, nt=NT, nq=NT - 1, K=3, W=3
            "value": n * nq / (ms * 1e-3), "unit": "interpolated rows/s", "ms": ms,
            "algorithmic_bytes": algo_bytes,
            "achieved_GBs": algo_bytes / (ms * 1e-3) / 1e9,
-           "gpu_launches": 4 * K}  # transpose, sweep, moments, evaluation
+           "gpu_launches": 2 * K}  # the grid's factors, rows to output
     if cpu:
         try:
             from scipy import interpolate as si
@@ -841,9 +842,9 @@ def methods_leg(gb, torch, dev, stream, pg, peak, rank, cpu=True, n=131072, K=3,
             except Exception as exc:  # report, do not hide
                 entry["cpu_reference"] = {"value": None, "error": repr(exc)}
         res["per_method"][m] = entry
-    # cost pass + orbit kernel per timed or warm-up run (the autotuner's trial
-    # launches come before)
-    res["gpu_launches"] = 2 * (K + W) * len(METHOD_FLOPS)
+    # cost pass + radial table + orbit kernel per timed or warm-up run (the
+    # autotuner's trial launches come before)
+    res["gpu_launches"] = 3 * (K + W) * len(METHOD_FLOPS)
     return res
 
 
