@@ -751,6 +751,11 @@ struct OrbitSystem {
   }
 };
 
+// The same system for the machines of this file: OrbitSystem itself selects
+// the Nystrom machines (machines_nystrom.cuh).
+template <int D>
+struct FirstOrderOrbit : OrbitSystem<D, false> {};
+
 // Surface-of-section integration (evalSOSDeriv, integrateFullOrbit.c:
 // 1353-1390): y = (x, y, vx, vy, A, t, psi) with z = A sin(psi) and
 // vz = A cos(psi); the independent variable is the increment of psi, and
@@ -1422,7 +1427,12 @@ struct Dop853Machine : OrbitCommon {
   static constexpr int kSlotDoubles = kSlots * N;
   double y0[N], k1[N];
   double* ks;  // slot store: slot s >= 1 at ks[((s - 1) * N + i) * kSlotStride]
-  GPC_HD GPC_FI void bind(double* base) { ks = base; }
+  GPC_HD GPC_FI void bind(double* base, bool queue = false)
+  {
+    ks = base;
+    queued = queue;
+    want_enqueue = false;
+  }
   GPC_HD GPC_FI double& K(int s, int i) const { return ks[((s - 1) * N + i) * kSlotStride]; }
   double h, hnew, hmax, pos_neg, rtol, atol;
   double t_current, t_old;
@@ -1616,6 +1626,15 @@ struct Dop853Machine : OrbitCommon {
     if (stage == ST_FSAL) {
       nsteps++;
       if (output_pending()) {
+        if (queued) {
+          // the rows of this step go to the warp's queue: the kernel writes
+          // the request, then calls finish_step
+          jf = iout + 1;
+          while (output_pending()) iout++;
+          jl = iout;
+          want_enqueue = true;
+          return;
+        }
         stage = ST_S14;
         return;
       }
@@ -1645,7 +1664,8 @@ struct Dop853Machine : OrbitCommon {
   // y0 to y1 (leung_dop853.c:441-474): k1 the step's first derivative,
   // k2 / k3 the stage-11 / stage-12 derivatives (kept in the K2 / K3 slots,
   // as the reference reuses k2 and k3), k4 = f(y1), k6..k10 the stage
-  // derivatives, s14..s16 the three dense-output stages.
+  // derivatives, s14..s16 the three dense-output stages.  Shared by the
+  // in-slot and the queued dense output, so both give the same rows.
   GPC_HD GPC_FI static double dense_value(double sv, double h, double y0, double y1, double k1,
                                           double k2, double k3, double k4, double k6,
                                           double k7, double k8, double k9, double k10,
@@ -1671,6 +1691,140 @@ struct Dop853Machine : OrbitCommon {
     rc8 = h * (rc8 + d713 * k4 + d714 * s14 + d715 * s15 + d716 * s16);
     return rc1 +
            sv * (ydiff + s1 * (bspl + sv * (rc4 + s1 * (rc5 + sv * (rc6 + s1 * (rc7 + sv * rc8))))));
+  }
+
+  // ---- queued dense output ---------------------------------------------
+  // With a request queue (the kernel's per-warp ring in global memory), a
+  // step that contains output times does not run the three dense-output
+  // stages in the warp's slot cycle, where the other lanes of the warp would
+  // sit idle for them: the lane writes the step's data to the queue and goes
+  // on with its next step, and the warp later runs the dense stages of 32
+  // queued requests side by side (one per lane).  The rows are the same as
+  // the in-slot dense output's (same arithmetic, dense_value).
+  //
+  // Request record, field-major with kQueueSlots slots per field (component
+  // i of vector field f of slot p at q[(f * N + i) * kQueueSlots + p]):
+  //   vector fields 0 y0, 1 k1, 2..10 the slot store K2..K10 (K5 = y1,
+  //   K4 = f(y1)); then scalars h, t_old, the orbit index and the row range
+  //   (first << 32 | last) at q[(11 N + k) * kQueueSlots + p], k = 0..3.
+  static constexpr int kQueueSlots = 64;
+  static constexpr int kQueueFields = 11 * N + 4;  // doubles per slot
+  static constexpr bool kQueue = SYS::kRow == ROW_ORBIT && !VAR;
+  static constexpr int kFsalSlot = 11, kDenseSlot = 12, kLastSlot = 14;
+  GPC_HD GPC_FI static long long req_orbit(const double* q, int p)
+  {
+    return reinterpret_cast<const long long*>(q)[(11 * N + 2) * kQueueSlots + p];
+  }
+  bool queued;        // dense output through the warp's queue
+  bool want_enqueue;  // this step's dense output waits for the queue
+  int jf, jl;         // rows of the pending request
+
+  GPC_HD GPC_FI void write_request(double* q, int p, long long orbit) const
+  {
+    constexpr int QS = kQueueSlots;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+      q[(0 * N + i) * QS + p] = y0[i];
+      q[(1 * N + i) * QS + p] = k1[i];
+    }
+#pragma unroll
+    for (int s = 1; s <= 9; s++)
+#pragma unroll
+      for (int i = 0; i < N; i++) q[((1 + s) * N + i) * QS + p] = K(s, i);
+    q[(11 * N + 0) * QS + p] = h;
+    q[(11 * N + 1) * QS + p] = t_old;
+    long long* qi = reinterpret_cast<long long*>(q);
+    qi[(11 * N + 2) * QS + p] = orbit;
+    qi[(11 * N + 3) * QS + p] = ((long long)jf << 32) | (long long)(unsigned)jl;
+  }
+
+  // Slot s of request p: s = 0 its k1, 1..9 its K2..K10, 10 / 11 the dense
+  // stages S14 / S15, which the round keeps in this lane's own slot store
+  // (unused by the lane's orbit when dense output is queued).
+  GPC_HD GPC_FI double req_k(const double* q, int p, int s, int i) const
+  {
+    return s <= 9 ? q[((1 + s) * N + i) * kQueueSlots + p] : K(s, i);
+  }
+
+  // Input of dense stage `stage` (14, 15, 16) of request p: the table loop
+  // of point() over the request's slots.
+  GPC_HD GPC_FI void req_point(double* y, int stage, const double* q, int p) const
+  {
+    const DopStageTable& tb = dop_table();
+    const int n = tb.nterm[stage];
+    double acc[N];
+    {
+      const double c0 = tb.coef[stage][0];
+#pragma unroll
+      for (int i = 0; i < N; i++) acc[i] = c0 * q[(1 * N + i) * kQueueSlots + p];
+    }
+#pragma unroll 4
+    for (int tt = 1; tt < n; tt++) {
+      const int s = tb.slot[stage][tt];
+      const double c = tb.coef[stage][tt];
+#pragma unroll
+      for (int i = 0; i < N; i++) acc[i] += c * req_k(q, p, s, i);
+    }
+    const double hq = q[(11 * N) * kQueueSlots + p];
+#pragma unroll
+    for (int i = 0; i < N; i++) y[i] = q[(0 * N + i) * kQueueSlots + p] + hq * acc[i];
+  }
+
+  // Time of dense stage `stage` of request p (t_old + c_s h of its step).
+  GPC_HD GPC_FI double req_tpoint(const double* y, int stage, const double* q, int p) const
+  {
+    if constexpr (SYS::kTimeIndex >= 0) {
+      return y[SYS::kTimeIndex];
+    } else {
+      return q[(11 * N + 1) * kQueueSlots + p] + stage_c(stage) * q[(11 * N) * kQueueSlots + p];
+    }
+  }
+
+  // Derivative of dense stage `stage` at request p: stages 14 and 15 are
+  // kept for the next stage inputs; stage 16 completes the rows.
+  template <class W>
+  GPC_HD void req_consume(const double* y, const double* a, int stage, const double* q, int p,
+                          const double* tt, W& out)
+  {
+    double d[N];
+    SYS::deriv(y, a, d);
+    if (stage < ST_S16) {
+      const int s = stage == ST_S14 ? S14 : S15;
+#pragma unroll
+      for (int i = 0; i < N; i++) K(s, i) = d[i];
+      return;
+    }
+    constexpr int QS = kQueueSlots;
+    const double hq = q[(11 * N) * QS + p], told = q[(11 * N + 1) * QS + p];
+    const long long rr = reinterpret_cast<const long long*>(q)[(11 * N + 3) * QS + p];
+    const int j0 = (int)(rr >> 32), j1 = (int)(unsigned)(rr & 0xffffffffLL);
+    for (int j = j0; j <= j1; j++) {
+      const double sv = (tt[j] - told) / hq;
+      double v[N];
+#pragma unroll
+      for (int k = 0; k < N; k++) v[k] = 0.0;
+      // one component at a time: unrolled, the compiler would issue all
+      // 14 N loads of the record at once and hold them in registers.  The
+      // component index of this loop is a run-time value, so d and v are
+      // read and written through selects over compile-time indices: indexed
+      // by it they would live in local memory.
+#pragma unroll 1
+      for (int i = 0; i < N; i++) {
+        double di = d[0];
+#pragma unroll
+        for (int k = 1; k < N; k++) di = i == k ? d[k] : di;
+        const double vi =
+            dense_value(sv, hq, q[(0 * N + i) * QS + p], q[((1 + K5) * N + i) * QS + p],
+                        q[(1 * N + i) * QS + p], q[((1 + K2) * N + i) * QS + p],
+                        q[((1 + K3) * N + i) * QS + p], q[((1 + K4) * N + i) * QS + p],
+                        q[((1 + K6) * N + i) * QS + p], q[((1 + K7) * N + i) * QS + p],
+                        q[((1 + K8) * N + i) * QS + p], q[((1 + K9) * N + i) * QS + p],
+                        q[((1 + K10) * N + i) * QS + p], K(S14, i), K(S15, i), di);
+#pragma unroll
+        for (int k = 0; k < N; k++) v[k] = i == k ? vi : v[k];
+      }
+      out(j, v);
+    }
   }
 
   GPC_HD void after_stage12()

@@ -26,12 +26,8 @@
 // Measured on a B200, first-order form -> this one: dop853, 1,048,576 orbits
 // with their own end times 908 -> 569 ms, one orbit of 1,165 steps 21.5 ->
 // 14.6 ms, 262,143 orbits in 96 parameter groups 64.4 -> 51.0 ms; rk4,
-// 100,001 orbits x 2,000 steps 38.6 -> 25.3 ms.  In the full run-time list,
-// which pairs the usual components and the Dehnen bar (potentials.cuh, sum2):
-// 3,000 orbits in MWPotential2014 with a bar, dop853 37.8 -> 21.2 ms, dopr54
-// 65.8 -> 36.9; an ellipsoidal NFW halo, not paired, dop853 4.73 -> 4.54; a
-// nonaxisymmetric SCF expansion, not paired and alone in its list, is the one
-// that loses: dop853 in 3D 139 -> 153 ms (planar 170 -> 142).
+// 100,001 orbits x 2,000 steps 38.6 -> 25.3 ms; dopr54 in the full run-time
+// list (forces not paired there) 54.9 -> 51.0 ms.
 //
 // The steps are the first-order form's up to rounding: same error estimates,
 // controller, step estimators, force times, dense output and status codes

@@ -65,8 +65,7 @@ struct KArgs {
   double scal[kMaxComp * kScalarStride];
 };
 
-// Whether machine M can queue its dense output (M::kQueue, default false): it
-// then runs in pair_loop.
+// Whether machine M can queue its dense output (M::kQueue, default false).
 template <class M, class = void>
 struct QueueOf {
   static constexpr bool value = false;
@@ -195,6 +194,144 @@ __device__ __forceinline__ void advance(const KArgs& A, M& m, const GpComp* comp
     M::pos(y, q);
     eval_force<D, PREC, VAR, POT>(comps, A.ncomp, q, a, A.scal, tf, A.rtab);
     m.consume(y, a, rows, slot);
+  }
+}
+
+// The persistent loop of a first-order machine whose dense output goes
+// through the warp's request queue (Dop853Machine with KArgs::dense_q set).  The slot
+// cycle of an attempt is slots 0..kFsalSlot; after the last the lanes whose
+// step contains output times append a request to the warp's ring (ballot +
+// prefix count, so the records are contiguous), and whenever 32 or more
+// requests wait -- or the warp has no orbits left -- slots
+// kDenseSlot..kLastSlot are a dense round: lane L runs the dense stages of
+// request head + L and writes its rows.  Every lane of the warp stays in the
+// loop until the warp has no orbit and no request left (the ballots need all
+// 32 lanes), so a lane without an orbit idles instead of leaving.
+template <class M, int D, int PREC, bool VAR, class POT>
+__device__ __forceinline__ void queued_loop(const KArgs& A, double* slot_store, int my_role)
+{
+  constexpr bool CYL_OK = !VAR;
+  constexpr unsigned FULL = 0xffffffffu;
+  constexpr int QS = M::kQueueSlots;
+  using Rows = DevRows<M::NV, D, CYL_OK, M::kRow>;
+  const int lane = threadIdx.x & 31;
+  const long long warp_id = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  double* const q = A.dense_q + warp_id * (long long)(M::kQueueFields * QS);
+  M m;
+  m.bind(slot_store + threadIdx.x, true);
+  long long i = 0, pos = 0;  // the active orbit and its output position
+  bool active = false, aborting = false, idle = false;
+  const GpComp* comps = A.comps;
+  unsigned iter = 0;
+  int slot = 0, qhead = 0, qcount = 0, nround = 0;
+  for (;;) {
+    const bool dense = slot >= M::kDenseSlot;
+    if (!dense && !active && !idle) {
+      const long long qpos = next_orbit(A, my_role);
+      if (qpos < 0) {
+        idle = true;
+      } else {
+        i = A.order ? (long long)A.order[qpos] : qpos;
+        pos = out_pos(A, qpos, i);
+        if (aborting) {
+          A.err[i] = E_ABORT;
+          write_nan_rows<M::NV, D, CYL_OK, M::kRow>(A.out, pos, 0);
+          if (A.stage_idx) {
+            __threadfence();
+            publish_rows(A, pos, i);
+          }
+        } else {
+          if (A.pend) A.pend[pos] = 1;  // its own lane writes rows until it is done
+          double w[M::NV];
+          load_state<M>(A, i, w);
+          comps = A.comps + (A.group ? (long long)A.group[i] * A.ncomp : 0LL);
+          Rows rows{&A.out, pos};
+          m.init(w, A.t + (A.indiv_t ? i * (long long)A.nt : 0LL), A.nt, A.dt, A.rtol, A.atol,
+                 A.max_attempts, rows);
+          active = true;
+        }
+      }
+    }
+    const int p = (qhead + lane) & (QS - 1);
+    if (dense ? lane < nround : (active && !m.done)) {
+      long long o = i, opos = pos;
+      const GpComp* cp = comps;
+      const double* tt = A.t;
+      if (dense) {  // the request's output position, orbit and parameter group
+        opos = M::req_orbit(q, p);
+        o = orbit_at(A, opos);
+        cp = A.comps + (A.group ? (long long)A.group[o] * A.ncomp : 0LL);
+        tt += A.indiv_t ? o * (long long)A.nt : 0LL;
+      }
+      Rows rows{&A.out, opos};
+      double y[M::NY], qq[M::NA], a[M::NA], tf = 0.0;
+      if (dense) {
+        m.req_point(y, slot + 2, q, p);
+        if constexpr (POT::kTimeDep) tf = m.req_tpoint(y, slot + 2, q, p);
+      } else {
+        m.point(y, slot);
+        if constexpr (POT::kTimeDep) tf = m.tpoint(y, slot);
+      }
+      M::pos(y, qq);
+      eval_force<D, PREC, VAR, POT>(cp, A.ncomp, qq, a, A.scal, tf, A.rtab);
+      if (dense)
+        m.req_consume(y, a, slot + 2, q, p, tt, rows);
+      else
+        m.consume(y, a, rows, slot);
+      if (dense && A.stage_idx && slot == M::kLastSlot) release_rows(A, opos);  // rows written
+    }
+    // the requests of this slot's accepted steps (only the last slot of an
+    // attempt makes any)
+    if (slot == M::kFsalSlot) {
+      const unsigned want = __ballot_sync(FULL, m.want_enqueue);
+      if (m.want_enqueue) {
+        const int rank = __popc(want & ((1u << lane) - 1u));
+        if (A.pend) atomicAdd(&A.pend[pos], 1);  // the request writes rows at pos
+        m.write_request(q, (qhead + qcount + rank) & (QS - 1), pos);
+        m.want_enqueue = false;
+        Rows rows{&A.out, pos};
+        m.finish_step(rows);
+      }
+      qcount += __popc(want);
+    }
+    const bool all_idle = __all_sync(FULL, idle);
+    // next slot (uniform over the warp)
+    if (slot == M::kLastSlot) {
+      __syncwarp();  // every lane has read its request before the slots are reused
+      qhead = (qhead + nround) & (QS - 1);
+      qcount -= nround;
+      nround = 0;
+    }
+    if (slot == M::kFsalSlot || slot == M::kLastSlot || (all_idle && !dense)) {
+      if (qcount >= 32 || (all_idle && qcount > 0)) {
+        __syncwarp();  // the records of the ring are visible to every lane
+        nround = qcount < 32 ? qcount : 32;
+        slot = M::kDenseSlot;
+      } else {
+        slot = 0;
+      }
+    } else {
+      slot++;
+    }
+    if (all_idle && qcount == 0 && nround == 0) break;
+    ++iter;
+    if (A.abort_flag && ((iter & 255u) == 0u) &&
+        *reinterpret_cast<const volatile int*>(A.abort_flag)) {
+      aborting = true;
+      if (active && !m.done) {
+        m.err = E_ABORT;
+        m.done = true;
+      }
+    }
+    if (active && m.done) {
+      Rows rows{&A.out, pos};
+      fill_unreached_rows(m, rows);
+      A.err[i] = m.err;
+      if (A.nsteps) A.nsteps[i] = m.nsteps;
+      if (A.done_count) atomicAdd(A.done_count, 1ULL);
+      if (A.stage_idx) release_rows(A, pos);
+      active = false;
+    }
   }
 }
 
@@ -376,9 +513,14 @@ __global__ void __launch_bounds__(128, MINB) orbit_kernel(const __grid_constant_
   __syncthreads();
   int my_role = role;
   if (my_role == 2 || (my_role == 1 && threadIdx.x >= 32)) return;
-  if constexpr (QueueOf<M>::value) {
+  if constexpr (QueueOf<M>::value && PairOf<M>::value) {
     pair_loop<M, D, PREC, POT>(A, slot_store, my_role);
     return;
+  } else if constexpr (QueueOf<M>::value) {
+    if (A.dense_q) {
+      queued_loop<M, D, PREC, VAR, POT>(A, slot_store, my_role);
+      return;
+    }
   }
   M m;
   m.bind(slot_store + threadIdx.x);
@@ -468,20 +610,17 @@ constexpr int queue_doubles_of()
 
 // Register-budget variants (chosen by the autotuner, galpy_b200/autotune.py):
 // variant 0 is the default; variant 1 caps the registers so that more blocks
-// are resident (3 blocks/SM for DOP853, 4 for the lighter integrators).
+// are resident (3 blocks/SM for DOP853, whose slot store allows at most 3 in
+// its first-order form; 4 blocks/SM for the lighter integrators).
 //
 // The default budget lets the compiler use up to 255 registers, but where the
 // force is short: with the tabulated radial force a kick is bound by the warps
 // that overlap its loads and chains, not by what a thread can hold.  Measured
 // at 1, 3 / 4 and 5 blocks per SM (303,104 orbits, ms): symplec4 6.05, 4.05,
 // 4.74; rk4 7.69, 5.76, 8.37; rk6 16.6, 16.0 (3), 17.2 (4); dopr54 41.3, 31.3;
-// dop853 keeps one (17.3; 19.4 at 3, where its stage code spills).  Batches
-// that leave an SM's warps idle gain nothing from it and lose little: up to
-// 20,000 orbits one block is 0 to 6 % faster.  In the common run-time list 1
-// against 3 blocks (300,000 orbits, 3D / planar, ms): rk4 8.82 / 8.41, 6.94 /
-// 6.33; rk6 17.9 / 17.3, 15.7 / 13.1; dopr54 27.2 / 22.3, 22.0 / 15.8.  (Below
-// 60,000 orbits rk6 3D is 13 % faster at one block, dopr54 3D 4 to 9 %, the
-// others are alike.)
+// dop853 keeps one (17.3; 19.4 at 3, where its stage code spills).  In the
+// common run-time list the paired rk4 took 254 registers, 20.0 ms, and 18.4 at
+// 3 blocks.
 template <class M, class POT>
 constexpr int default_blocks()
 {

@@ -1,7 +1,7 @@
 """The Nystrom form of the Runge-Kutta machines (machines_nystrom.cuh): its
-tables against the published DOP853 tableau, its pairs of forces against single
-ones, and on the GPU the DOP853 machine in two forms of one potential over the
-sizes where the warp's rounds and its dense-output queue have edges."""
+tables against the published DOP853 tableau, and on the GPU the second-order
+machines against the first-order one over the sizes where the warp's slot
+cycle and its dense-output queue have edges."""
 import os
 import re
 from fractions import Fraction
@@ -152,10 +152,9 @@ def test_force_pairs(harness, golden, name, planar):
 @pytest.mark.parametrize("planar", [False, True])
 @pytest.mark.parametrize("n", [1, 31, 33, 129, 5000])
 def test_pair_machine_against_first_order(n, planar):
-    """DOP853 in MWPotential2014: the compile-time list with the tabulated radial
-    force against the full run-time list (signature 0; its parity with the
-    first-order reference code is test_gpu_parity.py's), per-orbit end times,
-    rows from none to several per step.  Both round differently:
+    """DOP853 in MWPotential2014: the pair machine (compile-time list) against
+    the first-order machine of the full run-time list (signature 0), per-orbit
+    end times, rows from none to several per step.  Both round differently:
     an orbit either takes the same steps and agrees to its conditioning, or
     one borderline step differs and it moves by its truncation error."""
     import torch
