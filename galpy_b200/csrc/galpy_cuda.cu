@@ -323,8 +323,8 @@ static int launch_persistent(const galpy_cuda_launch* L, const KernelInfo& ki, K
     GPC_CUDA_TRY(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
   // slot-store machines: all of the unified L1/shared array as shared memory
   // for the register-capped variant and for blocks below 128, so that 3
-  // blocks' slot stores (3 x 66 KB for 3D DOP853) fit per SM; the hot
-  // potential tables are a few KB
+  // blocks' slot stores fit per SM (3D DOP853: 36 KB each, 66 KB in first-order
+  // form); the hot potential tables are a few KB
   // (the attribute belongs to the kernel, so it is set on every launch)
   if (smem > 0)
     GPC_CUDA_TRY(cudaFuncSetAttribute(

@@ -27,12 +27,14 @@
 // with their own end times 908 -> 569 ms, one orbit of 1,165 steps 21.5 ->
 // 14.6 ms, 262,143 orbits in 96 parameter groups 64.4 -> 51.0 ms; rk4,
 // 100,001 orbits x 2,000 steps 38.6 -> 25.3 ms; dopr54 in the full run-time
-// list (forces not paired there) 54.9 -> 51.0 ms.
+// list, which pairs the usual components and the Dehnen bar (potentials.cuh,
+// sum2), 3,000 orbits in MWPotential2014 with a bar 65.8 -> 36.9 ms.
 //
 // The steps are the first-order form's up to rounding: same error estimates,
 // controller, step estimators, force times, dense output and status codes
 // (references in machines.cuh).  Surfaces of section are first-order systems
-// and stay with machines.cuh.
+// and stay with machines.cuh, and so does dop853 in the full run-time list
+// (orbit_kernels_dop853.cu).
 #pragma once
 #include <type_traits>
 #include <utility>
@@ -1584,5 +1586,20 @@ struct Dop853Machine<D, VAR, OrbitSystem<D, VAR>> : PairMachine<D, VAR> {
     }
   }
 };
+
+// The dop853 machine of a component list.
+// The full run-time list keeps the first-order machine, whose sums are in
+// the reference's order.  It carries the potentials whose second
+// derivative jumps (the Dehnen bar at its radius): there the error
+// estimate of many steps is near 1, and the pair machine's rounding
+// decides some of them otherwise, which moves an orbit by 7e-10 where the
+// first-order machine keeps to 30 times its one-ulp response
+// (tests/test_gpu_timedep.py).  Pairs would take 21.2 ms instead of 38.4
+// for 3,000 orbits in MWPotential2014 with a bar, 4.54 instead of 4.77 in
+// an ellipsoidal halo, and 153 instead of 146 in a nonaxisymmetric SCF
+// expansion.
+template <int D, bool VAR, class POT>
+using Dop853For = std::conditional_t<POT::kFullList && !VAR,
+                                     Dop853Machine<D, VAR, FirstOrderOrbit<D>>, Dop853Machine<D, VAR>>;
 
 }  // namespace gpc

@@ -254,18 +254,17 @@ __device__ __forceinline__ void queued_loop(const KArgs& A, double* slot_store, 
     }
     const int p = (qhead + lane) & (QS - 1);
     if (dense ? lane < nround : (active && !m.done)) {
+      // (the rows' bounds and times are formed after the force: formed before,
+      // they are held across it, and the force of the full list has every
+      // register in use)
+      double y[M::NY], qq[M::NA], a[M::NA];
       long long o = i, opos = pos;
       const GpComp* cp = comps;
-      const double* tt = A.t;
+      double tf = 0.0;  // the force's time (read by time-dependent component lists only)
       if (dense) {  // the request's output position, orbit and parameter group
         opos = M::req_orbit(q, p);
         o = orbit_at(A, opos);
         cp = A.comps + (A.group ? (long long)A.group[o] * A.ncomp : 0LL);
-        tt += A.indiv_t ? o * (long long)A.nt : 0LL;
-      }
-      Rows rows{&A.out, opos};
-      double y[M::NY], qq[M::NA], a[M::NA], tf = 0.0;
-      if (dense) {
         m.req_point(y, slot + 2, q, p);
         if constexpr (POT::kTimeDep) tf = m.req_tpoint(y, slot + 2, q, p);
       } else {
@@ -273,12 +272,14 @@ __device__ __forceinline__ void queued_loop(const KArgs& A, double* slot_store, 
         if constexpr (POT::kTimeDep) tf = m.tpoint(y, slot);
       }
       M::pos(y, qq);
-      eval_force<D, PREC, VAR, POT>(cp, A.ncomp, qq, a, A.scal, tf, A.rtab);
-      if (dense)
-        m.req_consume(y, a, slot + 2, q, p, tt, rows);
-      else
+      eval_force<D, PREC, VAR, POT>(cp, A.ncomp, qq, a, A.scal, tf);
+      Rows rows{&A.out, opos};
+      if (dense) {
+        m.req_consume(y, a, slot + 2, q, p, A.t + (A.indiv_t ? o * (long long)A.nt : 0LL), rows);
+        if (A.stage_idx && slot == M::kLastSlot) release_rows(A, opos);  // its rows are written
+      } else {
         m.consume(y, a, rows, slot);
-      if (dense && A.stage_idx && slot == M::kLastSlot) release_rows(A, opos);  // rows written
+      }
     }
     // the requests of this slot's accepted steps (only the last slot of an
     // attempt makes any)
@@ -618,9 +619,13 @@ constexpr int queue_doubles_of()
 // that overlap its loads and chains, not by what a thread can hold.  Measured
 // at 1, 3 / 4 and 5 blocks per SM (303,104 orbits, ms): symplec4 6.05, 4.05,
 // 4.74; rk4 7.69, 5.76, 8.37; rk6 16.6, 16.0 (3), 17.2 (4); dopr54 41.3, 31.3;
-// dop853 keeps one (17.3; 19.4 at 3, where its stage code spills).  In the
-// common run-time list the paired rk4 took 254 registers, 20.0 ms, and 18.4 at
-// 3 blocks.
+// dop853 keeps one (17.3; 19.4 at 3, where its stage code spills).  Batches
+// that leave an SM's warps idle gain nothing from it and lose little: up to
+// 20,000 orbits one block is 0 to 6 % faster.  In the common run-time list 1
+// against 3 blocks (300,000 orbits, 3D / planar, ms): rk4 8.82 / 8.41, 6.94 /
+// 6.33; rk6 17.9 / 17.3, 15.7 / 13.1; dopr54 27.2 / 22.3, 22.0 / 15.8.  (Up to
+// 60,000 orbits rk6 3D is 13 % faster at one block, dopr54 3D 4 to 9 %, the
+// others are alike.)
 template <class M, class POT>
 constexpr int default_blocks()
 {

@@ -11,12 +11,7 @@ struct Dop853Methods {
   static KernelInfo pick(int method, int variant)
   {
     if (method != M_DOP853) return KernelInfo();
-    // The full run-time list evaluates its forces one at a time, so pairing
-    // them gains nothing there: it keeps the first-order machine.
-    if constexpr (POT::kFullList && !VAR)
-      return info_of<Dop853Machine<D, VAR, FirstOrderOrbit<D>>, D, PREC, VAR, POT>(variant);
-    else
-      return info_of<Dop853Machine<D, VAR>, D, PREC, VAR, POT>(variant);
+    return info_of<Dop853For<D, VAR, POT>, D, PREC, VAR, POT>(variant);
   }
 };
 

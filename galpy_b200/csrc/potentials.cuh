@@ -1290,7 +1290,7 @@ using MW14MixedPot = MixedPot<DIRECT, MIX, T_PSWC, T_MN, T_NFW>;
 // 40 % for the FP64 pipe (symplec4, 1,048,576 orbits).  The bulge and the halo
 // are both spherical, a = f(r^2) x, so a launch in one potential tabulates
 // their sum f once, on the device, before it integrates (radial_table_kernel,
-// ~5 us): each binade of r^2 in kRadSub intervals, each a polynomial of degree
+// 8.5 us): each binade of r^2 in kRadSub intervals, each a polynomial of degree
 // 7 in its local variable.  An evaluation is then one row of 64 bytes (four
 // 16-byte loads) and 8 double-precision operations in place of 91.
 //

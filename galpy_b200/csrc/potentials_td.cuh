@@ -243,7 +243,10 @@ struct CylParts {
   double FR, tq, R2, p2, Rp;
 };
 
-GPC_HD inline CylParts disk_pert_parts(const GpComp* __restrict__ cp, int type, double R,
+// (inlined by force, as spiral_accel: left to the compiler it is a call where a
+// file holds many kernels, and a call anywhere in the force costs dop853's
+// full-list kernel 5 % in potentials that never take it)
+GPC_HD GPC_FI CylParts disk_pert_parts(const GpComp* __restrict__ cp, int type, double R,
                                        double phi, double t)
 {
   double a[9];
@@ -499,7 +502,7 @@ GPC_HD inline Dual3<HESS> spiral_potential(const GpComp* __restrict__ cp, double
 
 // Acceleration (and K if K) of the spiral arms at (x, y, z), time t, R > 0.
 template <bool PLANAR>
-GPC_HD inline void spiral_accel(const GpComp* __restrict__ cp, double x, double y, double z,
+GPC_HD GPC_FI void spiral_accel(const GpComp* __restrict__ cp, double x, double y, double z,
                                 double t, double& ax, double& ay, double& az, double* K)
 {
   const double zz = PLANAR ? 0.0 : z;
