@@ -1948,35 +1948,58 @@ template <class M, class F, class W>
 GPC_HD void run_orbit_queued(M& m, F& force, W& out, double* q, const double* tt,
                              long long orbit)
 {
-  double q1[M::NA], q2[M::NA], a1[M::NA], a2[M::NA], vn[M::NA], t1, t2;
-  const auto eval2 = [&] {
-    force(q1, a1, t1);
-    force(q2, a2, t2);
-  };
-  while (!m.done) {  // the kernel's pair_loop, one lane
-    const bool start = m.stage < 0;
-    const int first = start ? M::kInitSlot : 0, last = start ? M::kInitSlot + 1 : M::kFsalSlot;
-    for (int slot = first; slot <= last; slot++) {
-      m.slot_point(q1, q2, slot, q, 0);
-      m.slot_times(t1, t2, slot, q, 0);
-      eval2();
-      m.slot_keep(a1, a2, slot);
-    }
-    if (start || !m.attempt_end(q2, a1, a2, vn)) continue;
-    if (m.output_pending()) {
-      int jf, jl;
-      m.rows_of_step(jf, jl);
-      m.write_request(q, 0, orbit, jf, jl, a1, a2, q2, vn);
-      m.finish_step(q2, vn, a2);
-      for (int slot = M::kDenseSlot; slot <= M::kLastSlot; slot++) {
+  if constexpr (PairOf<M>::value) {
+    double q1[M::NA], q2[M::NA], a1[M::NA], a2[M::NA], vn[M::NA], t1, t2;
+    const auto eval2 = [&] {
+      force(q1, a1, t1);
+      force(q2, a2, t2);
+    };
+    while (!m.done) {  // the kernel's pair_loop, one lane
+      const bool start = m.stage < 0;
+      const int first = start ? M::kInitSlot : 0, last = start ? M::kInitSlot + 1 : M::kFsalSlot;
+      for (int slot = first; slot <= last; slot++) {
         m.slot_point(q1, q2, slot, q, 0);
         m.slot_times(t1, t2, slot, q, 0);
         eval2();
         m.slot_keep(a1, a2, slot);
       }
-      m.req_rows(a1, q, 0, tt, out);
-    } else {
-      m.finish_step(q2, vn, a2);
+      if (start || !m.attempt_end(q2, a1, a2, vn)) continue;
+      if (m.output_pending()) {
+        int jf, jl;
+        m.rows_of_step(jf, jl);
+        m.write_request(q, 0, orbit, jf, jl, a1, a2, q2, vn);
+        m.finish_step(q2, vn, a2);
+        for (int slot = M::kDenseSlot; slot <= M::kLastSlot; slot++) {
+          m.slot_point(q1, q2, slot, q, 0);
+          m.slot_times(t1, t2, slot, q, 0);
+          eval2();
+          m.slot_keep(a1, a2, slot);
+        }
+        m.req_rows(a1, q, 0, tt, out);
+      } else {
+        m.finish_step(q2, vn, a2);
+      }
+    }
+  } else {  // the kernel's queued_loop, one lane
+    double y[M::NY], qq[M::NA], a[M::NA];
+    int slot = 0;
+    while (!m.done) {
+      m.point(y, slot);
+      M::pos(y, qq);
+      force(qq, a, m.tpoint(y, slot));
+      m.consume(y, a, out, slot);
+      if (slot == M::kFsalSlot && m.want_enqueue) {
+        m.write_request(q, 0, orbit);
+        m.want_enqueue = false;
+        m.finish_step(out);
+        for (int stage = M::kDenseSlot + 2; stage <= M::kLastSlot + 2; stage++) {
+          m.req_point(y, stage, q, 0);
+          M::pos(y, qq);
+          force(qq, a, m.req_tpoint(y, stage, q, 0));
+          m.req_consume(y, a, stage, q, 0, tt, out);
+        }
+      }
+      slot = slot == M::kFsalSlot ? 0 : slot + 1;
     }
   }
   fill_unreached_rows(m, out);

@@ -23,6 +23,17 @@ int records(int planar, int npot, const int* pot_type, const double* pot_args,
   return compile_group(planar, npot, pot_type, pot_args, comps.data(), nullptr);
 }
 
+bool is_mw14(int npot, const int* pot_type)
+{
+  return npot == 3 && pot_type[0] == T_PSWC && pot_type[1] == T_MN && pot_type[2] == T_NFW;
+}
+bool is_common(const std::vector<GpComp>& comps)
+{
+  for (const GpComp& c : comps)
+    if (needs_full_list(c.type)) return false;
+  return true;
+}
+
 struct Rows {
   double* out;
   int nv, nt;
@@ -81,7 +92,7 @@ int dispatch(int method, int nobj, const double* w, int nt, const double* t, int
     HARNESS_CASE(M_RK4, RKMachine<D, VAR, 4>)
     HARNESS_CASE(M_RK6, RKMachine<D, VAR, 6>)
     HARNESS_CASE(M_DOPR54, Dopr54Machine<D, VAR>)
-    HARNESS_CASE(M_DOP853, Dop853Machine<D, VAR>)
+    HARNESS_CASE(M_DOP853, Dop853For<D, VAR, POT>)
 #undef HARNESS_CASE
   }
   return -2;
@@ -98,23 +109,27 @@ extern "C" int harness_integrate(int planar, int var, int method, int prec, int 
   int rc = records(planar, npot, pot_type, pot_args, comps);
   if (rc) return rc;
   const GpComp* c = comps.data();
-  // the kernels' compile-time MWPotential2014 specialisation
-  const bool mw14 = npot == 3 && pot_type[0] == T_PSWC && pot_type[1] == T_MN &&
-                    pot_type[2] == T_NFW;
+  // the kernels' lists: MWPotential2014's at compile time, the common and the
+  // full run-time list (float32 forces and deviations: the full one)
+  const bool mw14 = is_mw14(npot, pot_type), common = is_common(comps);
   const int nrec = (int)comps.size();
 #define HARNESS_ARGS method, nobj, w, nt, t, indiv_t, c, nrec, dt, rtol, atol, max_att, out, err, nsteps
   if (var) return planar ? dispatch<2, PREC_FP64, true, DynPot>(HARNESS_ARGS)
                          : dispatch<3, PREC_FP64, true, DynPot>(HARNESS_ARGS);
-  if (planar) {
-    if (prec) return mw14 ? dispatch<2, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
-                          : dispatch<2, PREC_F32, false, DynPot>(HARNESS_ARGS);
-    return mw14 ? dispatch<2, PREC_FP64, false, MW14Pot>(HARNESS_ARGS)
-                : dispatch<2, PREC_FP64, false, DynPot>(HARNESS_ARGS);
+  if (prec) {
+    if (planar) return mw14 ? dispatch<2, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
+                            : dispatch<2, PREC_F32, false, DynPot>(HARNESS_ARGS);
+    return mw14 ? dispatch<3, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
+                : dispatch<3, PREC_F32, false, DynPot>(HARNESS_ARGS);
   }
-  if (prec) return mw14 ? dispatch<3, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
-                        : dispatch<3, PREC_F32, false, DynPot>(HARNESS_ARGS);
-  return mw14 ? dispatch<3, PREC_FP64, false, MW14Pot>(HARNESS_ARGS)
-              : dispatch<3, PREC_FP64, false, DynPot>(HARNESS_ARGS);
+  if (planar) {
+    if (mw14) return dispatch<2, PREC_FP64, false, MW14Pot>(HARNESS_ARGS);
+    return common ? dispatch<2, PREC_FP64, false, DynPotCommon>(HARNESS_ARGS)
+                  : dispatch<2, PREC_FP64, false, DynPot>(HARNESS_ARGS);
+  }
+  if (mw14) return dispatch<3, PREC_FP64, false, MW14Pot>(HARNESS_ARGS);
+  return common ? dispatch<3, PREC_FP64, false, DynPotCommon>(HARNESS_ARGS)
+                : dispatch<3, PREC_FP64, false, DynPot>(HARNESS_ARGS);
 #undef HARNESS_ARGS
 }
 
@@ -126,7 +141,7 @@ static void run_dop853_queued(int nobj, const double* w, int nt, const double* t
                               const GpComp* comps, int ncomp, double rtol, double atol,
                               long long max_att, double* out, int* err, long long* nsteps)
 {
-  using M = Dop853Machine<D, false>;
+  using M = Dop853For<D, false, POT>;
   Force<D, PREC_FP64, false, POT> f{comps, ncomp, {}};
   for (int k = 0; k < ncomp && k < kMaxComp; k++)
     for (int j = 0; j < kScalarStride; j++) f.scal[k * kScalarStride + j] = comps[k].c[j];
@@ -152,23 +167,19 @@ extern "C" int harness_dop853_queued(int planar, int nobj, const double* w, int 
   std::vector<GpComp> comps;
   int rc = records(planar, npot, pot_type, pot_args, comps);
   if (rc) return rc;
-  const bool mw14 = npot == 3 && pot_type[0] == T_PSWC && pot_type[1] == T_MN &&
-                    pot_type[2] == T_NFW;
+#define QUEUED_ARGS \
+  nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol, max_att, out, err, nsteps
+  const bool mw14 = is_mw14(npot, pot_type), common = is_common(comps);
   if (planar) {
-    if (mw14)
-      run_dop853_queued<2, MW14Pot>(nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol,
-                                    max_att, out, err, nsteps);
-    else
-      run_dop853_queued<2, DynPot>(nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol,
-                                   max_att, out, err, nsteps);
+    if (mw14) run_dop853_queued<2, MW14Pot>(QUEUED_ARGS);
+    else if (common) run_dop853_queued<2, DynPotCommon>(QUEUED_ARGS);
+    else run_dop853_queued<2, DynPot>(QUEUED_ARGS);
   } else {
-    if (mw14)
-      run_dop853_queued<3, MW14Pot>(nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol,
-                                    max_att, out, err, nsteps);
-    else
-      run_dop853_queued<3, DynPot>(nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol,
-                                   max_att, out, err, nsteps);
+    if (mw14) run_dop853_queued<3, MW14Pot>(QUEUED_ARGS);
+    else if (common) run_dop853_queued<3, DynPotCommon>(QUEUED_ARGS);
+    else run_dop853_queued<3, DynPot>(QUEUED_ARGS);
   }
+#undef QUEUED_ARGS
   return 0;
 }
 

@@ -1,7 +1,7 @@
 """The Nystrom form of the Runge-Kutta machines (machines_nystrom.cuh): its
-tables against the published DOP853 tableau, and on the GPU the second-order
-machines against the first-order one over the sizes where the warp's slot
-cycle and its dense-output queue have edges."""
+tables against the published DOP853 tableau, its pairs of forces against single
+ones, and on the GPU the second-order machines against the first-order one over
+the sizes where the warp's rounds and its dense-output queue have edges."""
 import os
 import re
 from fractions import Fraction
@@ -146,6 +146,27 @@ def test_force_pairs(harness, golden, name, planar):
                         want = np.concatenate([want, np.einsum("nij,nj->ni", K, q[:, D:])], 1)
                     # the same sums up to their order: a few roundings
                     assert np.abs(a - want).max() <= 1e-14 * np.abs(want).max(), (var, lst, t1, t2)
+
+
+@pytest.mark.parametrize("planar", [False, True])
+@pytest.mark.parametrize("name", ["bar_growing+mw14", "ell_trihern"])
+def test_full_list_queued_dense_output(harness, golden, name, planar):
+    """The full run-time list's dop853 machine, which is the first-order one:
+    rows from its request records against its own dense stages, bit for bit,
+    several rows a step and none, forward and backward."""
+    from helpers import cyl_to_rect, seeded_ics
+
+    if name in timedep_pots.NAMES:
+        pt, pa = timedep_pots.potential(name, planar=planar)
+    else:
+        key = name + "_planar" if planar else name
+        pt, pa = golden[key + "_type"], golden[key + "_args"]
+    w = cyl_to_rect(seeded_ics(6, 62, planar=planar))
+    for t in (np.linspace(0.0, 8.0, 161), np.linspace(0.0, -6.0, 5)):
+        ref = harness.integrate(w, t, pt, pa, "dop853", planar=planar, rtol=1e-10, atol=1e-10)
+        got = harness.dop853_queued(w, t, pt, pa, planar=planar, rtol=1e-10, atol=1e-10)
+        assert not ref[1].any()
+        assert all(np.array_equal(a, b) for a, b in zip(got, ref))
 
 
 @pytest.mark.gpu
