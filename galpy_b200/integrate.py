@@ -382,10 +382,10 @@ def integrate_device(comps, ncomp, w0, t, out, err, int_method, planar=False, va
     planar rows of 5, planar=True) with rk4/rk6/dopr54/dop853 in float64.
     Runs on `stream` (a torch.cuda.Stream, default: the current stream).
     abort_flag: optional int32 CUDA tensor (one element) that the kernel polls
-    every 256 loop iterations; once it reads non-zero, the orbits in flight
-    stop with err -10 and NaN rows after their last written one, and orbits
-    not yet started get err -10 and NaN rows (the device form of galpy's
-    SIGINT handling)."""
+    every 256 loop iterations (dop853: every 32 attempts); once it reads
+    non-zero, the orbits in flight stop with err -10 and NaN rows after their
+    last written one, and orbits not yet started get err -10 and NaN rows (the
+    device form of galpy's SIGINT handling)."""
     import torch
 
     layouts_in = {"aos": _lib.IN_AOS, "soa": _lib.IN_SOA}

@@ -51,7 +51,10 @@ extern "C" {
 /* precision of the force evaluation and the state.  FP64 and F32FORCE apply
  * to every method and potential; the three mixed forms to plain (not
  * variational) runs in MWPotential2014-type potentials
- * (GALPY_CUDA_SIG_MW14), other combinations return GALPY_CUDA_ERR_METHOD. */
+ * (GALPY_CUDA_SIG_MW14), other combinations return GALPY_CUDA_ERR_METHOD.
+ * In MWPotential2014 as one potential the float64 force is tabulated and
+ * faster than F64_TAIL32 and F32BULGE, which evaluate it directly (symplec4:
+ * 1, 0.61 and 0.73 of its speed); those two stay for callers that chose them. */
 #define GALPY_CUDA_FP64 0       /* float64 force and state */
 #define GALPY_CUDA_F32FORCE 1   /* float32 force, float64 state */
 #define GALPY_CUDA_F64_TAIL32 2 /* float64 force with the high-order terms of its special-
@@ -223,7 +226,7 @@ int integrateOrbit_dxdv_batch_cuda(int planar, int nobj, double *yo, int nt, dou
 /* Device-pointer entry point: all arrays live on the device, the call is
  * asynchronous on `stream`.  Its scratch is allocated stream-ordered per call
  * from the device's default pool: 128 bytes of control words, the scheduling
- * scratch (see `schedule`), dop853's dense-output requests (22 KB for each
+ * scratch (see `schedule`), dop853's dense-output requests (22 or 36 KB for each
  * resident warp) and, for MWPotential2014 as one potential with comps_host
  * set, the table of its radial force (246 KB). */
 typedef struct galpy_cuda_launch {
@@ -312,7 +315,10 @@ int galpy_cuda_jacobi_device(const void *comps, int ncomp, const int *group, int
  * (galpy's result layout); t [nt] or [n][nt] (indiv_t), increasing; tq [nq]
  * or [n][nq] (indiv_q); out [n][nq][nv].  Queries outside [t_0, t_end]
  * extrapolate the end pieces (galpy refuses them before it interpolates).
- * Device pointers, asynchronous on `stream`; scratch of 2*n*nt*nv doubles
+ * Device pointers, asynchronous on `stream`; on a shared grid of at least 4
+ * rows at most 5*nt doubles of scratch where the one-kernel form is the
+ * faster one (few orbits, or rows that leave a multiprocessor many orbits),
+ * else and with per-orbit grids scratch of 2*n*nt*nv doubles
  * (n*nt*nv below 4 rows; plus n*nt with per-orbit times) allocated
  * stream-ordered on it from the library's private memory pool (kept for the
  * next call; galpy_cuda_trim_memory returns it). */

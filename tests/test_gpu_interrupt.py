@@ -6,7 +6,8 @@ KeyboardInterrupt when any err is -10 (galpy/util/bovy_symplecticode.c:38-54,
 galpy/orbit/integrateFullOrbit.py:737-738); the reference tests this by
 sending SIGINT to a child process running a long integration
 (tests/test_orbit.py:12211-12420).  The engine forwards SIGINT to a device
-abort word that the persistent kernel polls every 256 loop iterations.
+abort word that the persistent kernel polls every 256 loop iterations (dop853:
+every 32 attempts).
 
 Nothing here faults or hangs a GPU: the interruption is a host-written flag
 (or a signal to a host process), and every kernel ends by itself.
