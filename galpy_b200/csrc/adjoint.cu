@@ -159,7 +159,7 @@ void launch_pass(Pass pass, int variant, const AdjK& K, unsigned blocks, unsigne
   }
 }
 
-using MW14Adj = FixedPot<false, T_PSWC, T_MN, T_NFW>;
+using MW14Adj = MW14GroupPot;
 
 int run_pass(Pass pass, const galpy_cuda_adjoint* a)
 {

@@ -1030,7 +1030,6 @@ GPC_HD GPC_FI bool usual_pair(const GpComp* __restrict__ cp, int type, PairPoint
 // and r^2 do not change under the rotation about z).  A KuzminLike frame
 // evaluates them at (xi, 0, 0) instead and adds fac a_x' grad xi.
 struct DynPot {
-  static constexpr bool kDirectScalars = false;
   static constexpr bool kAdditive = true;  // a component may add to a0
   static constexpr bool kTimeDep = true;
   static constexpr bool kPairList = true;  // sum2
@@ -1175,7 +1174,6 @@ struct DynPot {
 // registers (and some kernels a resident block): the host selects it for
 // potentials without such a component (GALPY_CUDA_SIG_COMMON).
 struct DynPotCommon {
-  static constexpr bool kDirectScalars = false;
   static constexpr bool kAdditive = true;
   static constexpr bool kTimeDep = false;
   static constexpr bool kPairList = true;  // sum2
@@ -1215,47 +1213,36 @@ struct DynPotCommon {
 };
 
 // Compile-time component list: the components are inlined side by side.
-// DIRECT: the scalars come from `scal` (kScalarStride doubles per component,
-// a kernel-parameter copy), else from the records in global memory.
-constexpr int kScalarStride = 16;
-template <bool DIRECT, int... TYPES>
+template <int... TYPES>
 struct FixedPot {
-  static constexpr bool kDirectScalars = DIRECT;
   static constexpr bool kAdditive =
       ((TYPES == T_HENONHEILES || TYPES == T_KUZMINDISK || is_ellipsoidal(TYPES)) || ...);
   static constexpr bool kTimeDep = false;
   static constexpr bool kInlinePair = true;  // two evaluations side by side (eval_force2)
   static constexpr bool kFullList = false;
   template <typename T, bool PLANAR>
-  GPC_HD GPC_FI static void sum(const GpComp* __restrict__ comp, const double* scal, int /*ncomp*/,
-                                T x, T y, T z, T z2, T R2, T r2, T& gR, T& gz, T& gyx,
-                                AddAcc<T>& a0, double /*t*/)
+  GPC_HD GPC_FI static void sum(const GpComp* __restrict__ comp, const double* /*scal*/,
+                                int /*ncomp*/, T x, T y, T z, T z2, T R2, T r2, T& gR, T& gz,
+                                T& gyx, AddAcc<T>& a0, double /*t*/)
   {
     int k = 0;
-    if (DIRECT) {
-      ((comp_accel<T, PLANAR, TYPES>(comp + k, ScalarsDirect{scal + kScalarStride * k}, x, y, z,
-                                     z2, R2, r2, gR, gz, gyx, a0, 0.0),
-        ++k),
-       ...);
-    } else {
-      ((comp_accel<T, PLANAR, TYPES>(comp + k, ScalarsGlobal{comp + k}, x, y, z, z2, R2, r2, gR,
-                                     gz, gyx, a0, 0.0),
-        ++k),
-       ...);
-    }
+    ((comp_accel<T, PLANAR, TYPES>(comp + k, ScalarsGlobal{comp + k}, x, y, z, z2, R2, r2, gR, gz,
+                                   gyx, a0, 0.0),
+      ++k),
+     ...);
   }
 };
-// galpy's MWPotential2014 order; MW14Pot takes the scalars as kernel
-// parameters (one potential per launch), MW14GroupPot from the records
-// (parameter groups).
-using MW14Pot = FixedPot<true, T_PSWC, T_MN, T_NFW>;
-using MW14GroupPot = FixedPot<false, T_PSWC, T_MN, T_NFW>;
+// galpy's MWPotential2014 order (parameter groups, variational runs and
+// gradients; one potential's plain runs take RadialPot).
+using MW14GroupPot = FixedPot<T_PSWC, T_MN, T_NFW>;
 
 // A compile-time list evaluated in one of the mixed float64 / float32 forms
 // (MIX_TAIL32, MIX_F32BULGE; float64 state and force accumulation).
+// DIRECT: the scalars come from `scal` (kScalarStride doubles per component,
+// a kernel-parameter copy), else from the records in global memory.
+constexpr int kScalarStride = 16;
 template <bool DIRECT, int MIX, int... TYPES>
 struct MixedPot {
-  static constexpr bool kDirectScalars = DIRECT;
   static constexpr bool kAdditive = false;
   static constexpr bool kTimeDep = false;
   static constexpr bool kInlinePair = true;
@@ -1389,7 +1376,6 @@ __device__ __forceinline__ float radial_evalf(const double* __restrict__ tab, fl
 // scalars from the kernel parameters, else from its record.
 template <bool DIRECT>
 struct RadialPot {
-  static constexpr bool kDirectScalars = DIRECT;
   static constexpr bool kAdditive = false;
   static constexpr bool kTimeDep = false;
   static constexpr bool kInlinePair = true;
@@ -1535,8 +1521,8 @@ template <class POT>
 struct IsMw14 {
   static constexpr bool value = false;
 };
-template <bool DIRECT>
-struct IsMw14<FixedPot<DIRECT, T_PSWC, T_MN, T_NFW>> {
+template <>
+struct IsMw14<MW14GroupPot> {
   static constexpr bool value = true;
 };
 struct Mw14Sphere {

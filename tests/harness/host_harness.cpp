@@ -117,17 +117,17 @@ extern "C" int harness_integrate(int planar, int var, int method, int prec, int 
   if (var) return planar ? dispatch<2, PREC_FP64, true, DynPot>(HARNESS_ARGS)
                          : dispatch<3, PREC_FP64, true, DynPot>(HARNESS_ARGS);
   if (prec) {
-    if (planar) return mw14 ? dispatch<2, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
+    if (planar) return mw14 ? dispatch<2, PREC_F32, false, MW14GroupPot>(HARNESS_ARGS)
                             : dispatch<2, PREC_F32, false, DynPot>(HARNESS_ARGS);
-    return mw14 ? dispatch<3, PREC_F32, false, MW14Pot>(HARNESS_ARGS)
+    return mw14 ? dispatch<3, PREC_F32, false, MW14GroupPot>(HARNESS_ARGS)
                 : dispatch<3, PREC_F32, false, DynPot>(HARNESS_ARGS);
   }
   if (planar) {
-    if (mw14) return dispatch<2, PREC_FP64, false, MW14Pot>(HARNESS_ARGS);
+    if (mw14) return dispatch<2, PREC_FP64, false, MW14GroupPot>(HARNESS_ARGS);
     return common ? dispatch<2, PREC_FP64, false, DynPotCommon>(HARNESS_ARGS)
                   : dispatch<2, PREC_FP64, false, DynPot>(HARNESS_ARGS);
   }
-  if (mw14) return dispatch<3, PREC_FP64, false, MW14Pot>(HARNESS_ARGS);
+  if (mw14) return dispatch<3, PREC_FP64, false, MW14GroupPot>(HARNESS_ARGS);
   return common ? dispatch<3, PREC_FP64, false, DynPotCommon>(HARNESS_ARGS)
                 : dispatch<3, PREC_FP64, false, DynPot>(HARNESS_ARGS);
 #undef HARNESS_ARGS
@@ -171,11 +171,11 @@ extern "C" int harness_dop853_queued(int planar, int nobj, const double* w, int 
   nobj, w, nt, t, indiv_t, comps.data(), (int)comps.size(), rtol, atol, max_att, out, err, nsteps
   const bool mw14 = is_mw14(npot, pot_type), common = is_common(comps);
   if (planar) {
-    if (mw14) run_dop853_queued<2, MW14Pot>(QUEUED_ARGS);
+    if (mw14) run_dop853_queued<2, MW14GroupPot>(QUEUED_ARGS);
     else if (common) run_dop853_queued<2, DynPotCommon>(QUEUED_ARGS);
     else run_dop853_queued<2, DynPot>(QUEUED_ARGS);
   } else {
-    if (mw14) run_dop853_queued<3, MW14Pot>(QUEUED_ARGS);
+    if (mw14) run_dop853_queued<3, MW14GroupPot>(QUEUED_ARGS);
     else if (common) run_dop853_queued<3, DynPotCommon>(QUEUED_ARGS);
     else run_dop853_queued<3, DynPot>(QUEUED_ARGS);
   }
